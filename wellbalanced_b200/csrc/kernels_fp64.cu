@@ -25,18 +25,22 @@ __global__ void primitive_fp64_kernel(const double* __restrict__ rho, const doub
   const int i = int(t / (Y + 1));
   const int j = int(t % (Y + 1));
   const int A = Y + 1;  // row pitch of az
-  if (j < Y) bxf[int64_t(i) * Y + j] = (az[int64_t(i) * A + j + 1] - az[int64_t(i) * A + j]) / dy + b0x;
-  if (i < X) byf[int64_t(i) * (Y + 1) + j] = -(az[int64_t(i + 1) * A + j] - az[int64_t(i) * A + j]) / dx + b0y;
+  using M = Math<double>;
+  const double idx = M::inv(dx), idy = M::inv(dy);
+  if (j < Y) bxf[int64_t(i) * Y + j] = M::div(az[int64_t(i) * A + j + 1] - az[int64_t(i) * A + j], dy, idy) + b0x;
+  if (i < X)
+    byf[int64_t(i) * (Y + 1) + j] = -M::div(az[int64_t(i + 1) * A + j] - az[int64_t(i) * A + j], dx, idx) + b0y;
   if (i >= X || j >= Y) return;
   const int64_t c = int64_t(i) * Y + j;
-  const double bx_lo = (az[int64_t(i) * A + j + 1] - az[int64_t(i) * A + j]) / dy + b0x;
-  const double bx_hi = (az[int64_t(i + 1) * A + j + 1] - az[int64_t(i + 1) * A + j]) / dy + b0x;
-  const double by_lo = -(az[int64_t(i + 1) * A + j] - az[int64_t(i) * A + j]) / dx + b0y;
-  const double by_hi = -(az[int64_t(i + 1) * A + j + 1] - az[int64_t(i) * A + j + 1]) / dx + b0y;
+  const double bx_lo = M::div(az[int64_t(i) * A + j + 1] - az[int64_t(i) * A + j], dy, idy) + b0x;
+  const double bx_hi = M::div(az[int64_t(i + 1) * A + j + 1] - az[int64_t(i + 1) * A + j], dy, idy) + b0x;
+  const double by_lo = -M::div(az[int64_t(i + 1) * A + j] - az[int64_t(i) * A + j], dx, idx) + b0y;
+  const double by_hi = -M::div(az[int64_t(i + 1) * A + j + 1] - az[int64_t(i) * A + j + 1], dx, idx) + b0y;
   const double r = rho[c];
-  const double u = mx[c] / r;
-  const double v = my[c] / r;
-  const double w = mz[c] / r;
+  const double ir = M::inv(r);
+  const double u = M::div(mx[c], r, ir);
+  const double v = M::div(my[c], r, ir);
+  const double w = M::div(mz[c], r, ir);
   const double bx = 0.5 * (bx_lo + bx_hi);
   const double by = 0.5 * (by_lo + by_hi);
   const double b = bz[c];
@@ -157,16 +161,18 @@ __global__ void rate_fp64_kernel(const double* __restrict__ rho, const double* _
     const int A = Y + 1;
     const int64_t c = int64_t(i) * Y + j;
     const double r = rho[c];
-    const double u = mx[c] / r, v = my[c] / r, w = mz[c] / r;
-    const double bx = 0.5 * ((az[int64_t(i) * A + j + 1] - az[int64_t(i) * A + j]) / dy + b0x +
-                             ((az[int64_t(i + 1) * A + j + 1] - az[int64_t(i + 1) * A + j]) / dy + b0x));
-    const double by = 0.5 * (-(az[int64_t(i + 1) * A + j] - az[int64_t(i) * A + j]) / dx + b0y +
-                             (-(az[int64_t(i + 1) * A + j + 1] - az[int64_t(i) * A + j + 1]) / dx + b0y));
+    using M = Math<double>;
+    const double ir = M::inv(r), idx = M::inv(dx), idy = M::inv(dy);
+    const double u = M::div(mx[c], r, ir), v = M::div(my[c], r, ir), w = M::div(mz[c], r, ir);
+    const double bx = 0.5 * (M::div(az[int64_t(i) * A + j + 1] - az[int64_t(i) * A + j], dy, idy) + b0x +
+                             (M::div(az[int64_t(i + 1) * A + j + 1] - az[int64_t(i + 1) * A + j], dy, idy) + b0x));
+    const double by = 0.5 * (-M::div(az[int64_t(i + 1) * A + j] - az[int64_t(i) * A + j], dx, idx) + b0y +
+                             (-M::div(az[int64_t(i + 1) * A + j + 1] - az[int64_t(i) * A + j + 1], dx, idx) + b0y));
     const double bzc = bz[c];
     const double p =
         (gamma - 1.0) * (energy[c] - 0.5 * r * (u * u + v * v + w * w) - 0.5 * (bx * bx + by * by + bzc * bzc));
-    rate = (fabs(u) + fast_speed(r, p, bx, by, bzc, gamma)) / dx +
-           (fabs(v) + fast_speed(r, p, by, bx, bzc, gamma)) / dy;
+    rate = M::div(fabs(u) + fast_speed(r, p, bx, by, bzc, gamma), dx, idx) +
+           M::div(fabs(v) + fast_speed(r, p, by, bx, bzc, gamma), dy, idy);
     smallest = r;
   }
   block_reduce_keys(rate, smallest, keys);
