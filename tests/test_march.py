@@ -1,0 +1,37 @@
+"""The 3D stage kernel's work list: marches shortened where few columns would leave SMs idle."""
+
+import numpy as np
+import pytest
+
+from wellbalanced_b200.mesh import AMRHierarchy, Layout
+
+
+def _covered(layout):
+    """How often the tiles of a layout cover each computed cell / node plane of its patches."""
+    counts = []
+    ty, tz = layout.tile_shape
+    for index, size in enumerate(layout._extents().tolist()):
+        count = np.zeros(size, dtype=int)
+        for t in layout.tiles[layout.tiles["patch"] == index]:
+            x, y, z = int(t["x0"]), int(t["y0"]), int(t["z0"])
+            count[x : x + layout.march, y : y + ty, z : z + tz] += 1
+        counts.append(count)
+    return counts
+
+
+@pytest.mark.parametrize("shape", [(4, 4, 4), (7, 5, 33), (64, 64, 64), (150, 97, 75), (256, 256, 256)])
+@pytest.mark.parametrize("lx", [3, 5, 32])
+def test_every_cell_lies_in_one_tile(shape, lx):
+    layout = Layout(AMRHierarchy(shape, periodic=(True, False, True)), precision=32, lx=lx)
+    assert 1 <= layout.march <= lx
+    for count in _covered(layout):
+        assert np.all(count == 1)
+
+
+def test_merged_parts_share_one_march():
+    parts = [Layout(AMRHierarchy(s, periodic=(True,) * 3), precision=64) for s in ((24,) * 3, (64,) * 3, (160, 96, 96))]
+    assert len({part.march for part in parts}) > 1
+    merged = Layout.merge(parts)
+    assert merged.march == min(part.march for part in parts)
+    for count in _covered(merged):
+        assert np.all(count == 1)

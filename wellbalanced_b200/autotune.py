@@ -30,6 +30,7 @@ def _key(engine):
 def _set_lx(engine, lx):
     layout = engine.layout
     layout.lx = int(lx)
+    layout.exact_march = True
     layout._tiles()
     from wellbalanced_b200.engine import _device_bytes
 

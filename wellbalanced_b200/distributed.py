@@ -208,6 +208,7 @@ class RankLayout:
         self.groups = layout.groups
         self.precision = layout.precision
         self.lx = layout.lx
+        self.march = layout.march
         self.tile_shape = layout.tile_shape
         self.default_tile = getattr(layout, "default_tile", layout.tile_shape)
         self.walls = layout.walls

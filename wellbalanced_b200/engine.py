@@ -260,12 +260,12 @@ class Engine:
             _lib.call("wb_stage3d_physics", self.precision, src.data_ptr(),
                       None if base is None else base.data_ptr(), dst.data_ptr(), self.patches.data_ptr(),
                       self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(), self.gamma, b[0], b[1], b[2],
-                      self.limiter, self.layout.lx, *self.physics, self.bad.data_ptr(), s)
+                      self.limiter, self.layout.march, *self.physics, self.bad.data_ptr(), s)
         else:
             ty, tz = self.layout.tile_shape
             _lib.call("wb_stage3d_tiled", self.precision, src.data_ptr(), None if base is None else base.data_ptr(),
                       dst.data_ptr(), self.patches.data_ptr(), self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(),
-                      self.gamma, b[0], b[1], b[2], self.limiter, self.layout.lx, ty, tz, self.bad.data_ptr(),
+                      self.gamma, b[0], b[1], b[2], self.limiter, self.layout.march, ty, tz, self.bad.data_ptr(),
                       None if bflux is None else bflux.data_ptr(), s)
         if timing:
             end.record(torch.cuda.current_stream(self.device) if self.stream is None else self.stream)

@@ -174,10 +174,12 @@ def _boxes_intersect(a, b):
     return tuple(out)
 
 
+#: SMs of a B200
+SMS = 148
 #: largest op the host builds (points); `size_ops` cuts a list further when it is small
 OP_MAX_POINTS = 1024
 #: op blocks resident on a B200 at once (148 SMs x 32 blocks of 64 threads)
-OP_WAVE = 148 * 32
+OP_WAVE = SMS * 32
 
 
 def op_points(total):
@@ -389,7 +391,10 @@ class Layout:
         self.nfields = 7 if self.ndim == 2 else 8
         self.groups = field_groups(self.ndim)
         self.precision = precision
+        #: 3D: cell planes of the stage kernel's x-march at most (`march` is what the tiles have)
         self.lx = lx
+        #: True where a caller has chosen the march itself (the autotuner): `march` is `lx`
+        self.exact_march = False
         #: 2D: the (tx, ty) tile shape of the stage kernel's work list (None: the default)
         self.tile = None if tile is None else tuple(int(v) for v in tile)
         self.walls = walls or ((False, False),) * self.ndim
@@ -552,23 +557,49 @@ class Layout:
         self._cut_tiles()
 
     def _cut_tiles(self):
-        """The stage kernel's work list: every patch's computed cells and nodes in tiles."""
-        tiles = []
-        for index in range(self.npatches):
-            n = [int(v) for v in self.rows[index]["n"]]
-            own = [n[a] + (1 if self.own[index][a] else 0) for a in range(self.ndim)]
-            if self.ndim == 2:
-                tx, ty = self.tile_shape
-                for x0 in range(0, own[0], tx):
-                    for y0 in range(0, own[1], ty):
-                        tiles.append((index, x0, y0, 0))
-            else:
-                ty, tz = self.tile_shape
-                for x0 in range(0, own[0], self.lx):
-                    for y0 in range(0, own[1], ty):
-                        for z0 in range(0, own[2], tz):
-                            tiles.append((index, x0, y0, z0))
-        self.tiles = np.array(tiles, dtype=np.int32).view(_lib.TILE).reshape(-1) if tiles else np.zeros(0, _lib.TILE)
+        """The stage kernel's work list: every patch's computed cells and nodes in tiles (3D:
+        columns of `march` cell planes)."""
+        self.march = self.lx if self.ndim == 2 or self.exact_march else self._short_march()
+        self.tiles = self._tiles_of(self.march)
+
+    def _extents(self):
+        """Cells and owned upper node planes of every patch (patches x axes)."""
+        own = np.array(self.own, dtype=np.int64).reshape(self.npatches, self.ndim)
+        return self.rows["n"][:, : self.ndim].astype(np.int64) + own
+
+    def _tiles_of(self, march):
+        a, b = self.tile_shape
+        steps = (a, b) if self.ndim == 2 else (march, a, b)
+        tiles = [(index, *origin, *(0,) * (3 - self.ndim))
+                 for index, size in enumerate(self._extents().tolist())
+                 for origin in itertools.product(*(range(0, n, step) for n, step in zip(size, steps, strict=True)))]
+        return np.array(tiles, dtype=np.int32).view(_lib.TILE).reshape(-1) if tiles else np.zeros(0, _lib.TILE)
+
+    def _short_march(self):
+        """Cell planes per tile: `lx`, or the halving of it (4 at least) that finishes earliest
+        where few columns leave SMs idle. A tile of L planes costs about L + 2.5 (its first
+        planes are loads and half the faces only), and an SM works through ceil(tiles / SMs) of
+        them, the longest among them; a shorter march has to win 2%. B200, before -> after:
+        64^3 float64 (16 columns) 389 -> 123 us a launch at 8 planes, 150 x 97 x 75 mixed
+        303 -> 259 us at 8, the 203-patch 64^3 multi-blast 269 -> 157 us at 8; 256^3 keeps 32
+        (2014 us; 16: 2104, 8: 2312)."""
+        size = self._extents()
+        if size.size == 0:
+            return self.lx
+        a, b = self.tile_shape
+        columns = -(-size[:, 1] // a) * -(-size[:, 2] // b)
+        best, cost = self.lx, None
+        march = self.lx
+        while march >= 4 or march == self.lx:
+            tiles = -(-size[:, 0] // march)
+            count = int((tiles * columns).sum())
+            planes = float((columns * (size[:, 0] + 2.5 * tiles)).sum()) / count
+            longest = min(march, int(size[:, 0].max())) + 2.5
+            found = longest + (-(-count // SMS) - 1) * planes
+            if cost is None or found < 0.98 * cost:
+                best, cost = march, found
+            march //= 2
+        return best
 
     def _chunks(self, per=2048):
         patch, start = [], []
@@ -885,6 +916,9 @@ class Layout:
         out.tile = getattr(first, "tile", None)
         out.default_tile = getattr(first, "default_tile", first.tile_shape)
         out.walls = first.walls
+        # one march for all parts: the kernel takes it per launch
+        out.march = min(part.march for part in layouts)
+        out.exact_march = True
         rows, tiles, chunk_patch, chunk_start, inv, inv_levels = [], [], [], [], [], []
         same_levels, boundary_levels, interp_levels = {}, {}, {}
         restrict_levels, face_ops = {}, []
@@ -898,7 +932,7 @@ class Layout:
             rows.append(r)
             own.extend(part.own)
             instances.extend([k] * part.npatches)
-            t = part.tiles.copy()
+            t = part.tiles.copy() if part.march == out.march else part._tiles_of(out.march)
             t["patch"] += patch_shift
             tiles.append(t)
             chunk_patch.append(part.chunk_patch + patch_shift)
