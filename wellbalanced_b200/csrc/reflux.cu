@@ -189,37 +189,12 @@ struct FacePhysics {
 template <typename S, typename R, int LIM, bool PHYS>
 __device__ void face_flux(const S* src, const PatchDesc& P, int ndim, int axis, int i, int j, int k,
                           const double* b0, double gamma, const FacePhysics& phys, double (&out)[6]) {
-  int comp[7], rows[6];
-  int ncons;
-  if (ndim == 2) {
-    ncons = 6;
-    if (axis == 0) {
-      const int c[7] = {0, 1, 2, 3, 4, 6, 7};
-      const int r[6] = {0, 1, 2, 3, 4, 6};
-      for (int t = 0; t < 7; ++t) comp[t] = c[t];
-      for (int t = 0; t < 6; ++t) rows[t] = r[t];
-    } else {
-      const int c[7] = {0, 2, 1, 3, 4, 5, 7};
-      const int r[6] = {0, 2, 1, 3, 4, 6};
-      for (int t = 0; t < 7; ++t) comp[t] = c[t];
-      for (int t = 0; t < 6; ++t) rows[t] = r[t];
-    }
-  } else {
-    ncons = 5;
-    const int s = axis, b = (axis + 1) % 3, c = (axis + 2) % 3;
-    comp[0] = 0;
-    comp[1] = 1 + s;
-    comp[2] = 1 + b;
-    comp[3] = 1 + c;
-    comp[4] = 4;
-    comp[5] = 5 + b;
-    comp[6] = 5 + c;
-    rows[0] = 0;
-    rows[1 + s] = 1;
-    rows[1 + b] = 2;
-    rows[1 + c] = 3;
-    rows[4] = 4;
-  }
+  // the frame of the face: 2D (x, y, z) and (y, x, z), 3D cyclic. Selects, not index tables:
+  // a component index that depends on the axis would put the states in local memory
+  const bool flat = ndim == 2;
+  auto normal = [&](R x, R y, R z) { return axis == 0 ? x : (axis == 1 ? y : z); };
+  auto first = [&](R x, R y, R z) { return axis == 0 ? y : (axis == 1 ? (flat ? x : z) : x); };
+  auto second = [&](R x, R y, R z) { return axis == 0 ? z : (axis == 1 ? (flat ? z : x) : y); };
   R qs[4][7];
   R bn = R(0);
 #pragma unroll
@@ -231,7 +206,13 @@ __device__ void face_flux(const S* src, const PatchDesc& P, int ndim, int axis, 
     R q[8], bl;
     cell_primitive<S, R>(src, P, ndim, ii, jj, kk, axis, b0, gamma, q, bl);
     if (st == 2) bn = bl;  // the face is the lower face of the third cell
-    for (int t = 0; t < 7; ++t) qs[st][t] = q[comp[t]];
+    qs[st][0] = q[0];
+    qs[st][1] = normal(q[1], q[2], q[3]);
+    qs[st][2] = first(q[1], q[2], q[3]);
+    qs[st][3] = second(q[1], q[2], q[3]);
+    qs[st][4] = q[4];
+    qs[st][5] = first(q[5], q[6], q[7]);
+    qs[st][6] = second(q[5], q[6], q[7]);
   }
   R L[7], Rt[7], F[7];
   reconstruct<LIM>(qs[0], qs[1], qs[2], qs[3], L, Rt);
@@ -268,56 +249,64 @@ __device__ void face_flux(const S* src, const PatchDesc& P, int ndim, int axis, 
   if (PHYS && ndim == 3 && phys.eta != 0.0) {
     F[4] += resistive_energy3<S, R>(src, P, axis, Cell3{{i, j, k}}, b0, R(phys.eta));
   }
-  for (int t = 0; t < ncons; ++t) out[t] = double(F[rows[t]]);
+  // back to (rho, m_x, m_y, m_z, E[, B_z])
+  out[0] = double(F[0]);
+  out[1] = double(axis == 0 ? F[1] : (axis == 1 ? (flat ? F[2] : F[3]) : F[2]));
+  out[2] = double(axis == 0 ? F[2] : (axis == 1 ? F[1] : F[3]));
+  out[3] = double(axis == 0 ? F[3] : (axis == 1 ? (flat ? F[3] : F[2]) : F[1]));
+  out[4] = double(F[4]);
+  if (flat) out[5] = double(F[6]);
 }
 
-// One warp per interface side: reg[slot] += mean of the fine faces over each coarse face -
-// the coarse face (each op holds both sides, so no two warps share a slot). The coarse face
-// and its 2 (2D) or 4 (3D) fine faces are evaluated by separate lanes (32 / K coarse faces
-// per round), then one lane per coarse face combines them from shared memory, the fine
-// faces summed in the order (a, b). Most interfaces are a few coarse faces long, so a warp
-// (four ops per 128-thread block) keeps the lanes busy where a block per op would not.
+// `splits` warps per interface side: reg[slot] += mean of the fine faces over each coarse
+// face - the coarse face (each op holds both sides, so no two warps share a slot). The
+// coarse face and its 2 (2D) or 4 (3D) fine faces are evaluated by separate lanes (32 / K
+// coarse faces per round), then one lane per coarse face combines them from shared memory,
+// the fine faces summed in the order (a, b). A face is a long chain of dependent loads and
+// arithmetic (~10 us), so what bounds the launch is the longest list of rounds one warp
+// walks: most interfaces are one or two rounds, but a 3D interface of 13 x 14 coarse faces
+// is 31. `flux_splits` spreads each op over as many warps as fill the SMs; a warp past the
+// end of its op leaves at once. B200, 1212 interfaces of up to 182 faces (3D multi-blast):
+// 316 us with one warp per op and the states in local memory, 43 us now.
 constexpr int kFluxThreads = 128;
 constexpr int kFluxWarps = kFluxThreads / 32;
+
+// Warps per op: 64 per SM in all (2 to 3 times what is resident, so that warps which leave
+// at once are replaced), at most 32.
+inline int flux_splits(int nops) { return max(1, min(32, 148 * 64 / max(nops, 1))); }
 
 template <typename S, typename R, int LIM, bool PHYS>
 __global__ void __launch_bounds__(kFluxThreads) face_flux_ops_kernel(const S* __restrict__ pool,
                                                                      const PatchDesc* __restrict__ patches,
                                                                      const FaceFluxOp* __restrict__ ops, int nops,
-                                                                     double b0x, double b0y, double b0z, double gamma,
+                                                                     int splits, double b0x, double b0y, double b0z, double gamma,
                                                                      FacePhysics phys, double* __restrict__ reg) {
   __shared__ double g_all[kFluxWarps][32][6];
   const int warp = threadIdx.x / 32, t = threadIdx.x % 32;
-  const int index = blockIdx.x * kFluxWarps + warp;
+  const int item = blockIdx.x * kFluxWarps + warp, index = item / splits;
   if (index >= nops) return;  // a whole warp: no block-wide barrier follows
   double(*g)[6] = g_all[warp];
   const FaceFluxOp op = ops[index];
-  const PatchDesc C = patches[op.coarse];
-  const PatchDesc F = patches[op.fine];
   const double b0[3] = {b0x, b0y, b0z};
   const int ncons = op.ndim == 2 ? 6 : 5;
   const int fine_b = op.ndim == 3 ? 2 : 1;
   const int K = 1 + 2 * fine_b;  // evaluations per coarse face
   const int per = 32 / K;        // coarse faces per round
   const int e = t % K;
-  for (int s0 = 0; s0 < op.len; s0 += per) {
+  for (int s0 = (item - index * splits) * per; s0 < op.len; s0 += per * splits) {
     const int s = s0 + t / K;
     if (t < per * K && s < op.len) {
       const int s1 = s / op.width, s2 = s % op.width;
-      int idx[3] = {0, 0, 0};
       double out[6] = {0, 0, 0, 0, 0, 0};
-      if (e == 0) {
-        idx[op.axis] = op.coarse_plane;
-        idx[op.t1] = op.coarse_t0[0] + s1;
-        if (op.ndim == 3) idx[op.t2] = op.coarse_t0[1] + s2;
-        face_flux<S, R, LIM, PHYS>(pool + C.off, C, op.ndim, op.axis, idx[0], idx[1], idx[2], b0, gamma, phys, out);
-      } else {
-        const int a = (e - 1) / fine_b, b = (e - 1) % fine_b;
-        idx[op.axis] = op.fine_plane;
-        idx[op.t1] = op.fine_t0[0] + 2 * s1 + a;
-        if (op.ndim == 3) idx[op.t2] = op.fine_t0[1] + 2 * s2 + b;
-        face_flux<S, R, LIM, PHYS>(pool + F.off, F, op.ndim, op.axis, idx[0], idx[1], idx[2], b0, gamma, phys, out);
-      }
+      // lane e: the coarse face (0) or one of the fine faces over it, one evaluation for both
+      const bool coarse = e == 0;
+      const int a = (e - 1) / fine_b, b = (e - 1) % fine_b;
+      const int plane = coarse ? op.coarse_plane : op.fine_plane;
+      const int u = coarse ? op.coarse_t0[0] + s1 : op.fine_t0[0] + 2 * s1 + a;
+      const int v = op.ndim == 2 ? 0 : (coarse ? op.coarse_t0[1] + s2 : op.fine_t0[1] + 2 * s2 + b);
+      auto at = [&](int axis) { return axis == op.axis ? plane : (axis == op.t1 ? u : v); };
+      const PatchDesc Q = patches[coarse ? op.coarse : op.fine];
+      face_flux<S, R, LIM, PHYS>(pool + Q.off, Q, op.ndim, op.axis, at(0), at(1), at(2), b0, gamma, phys, out);
 #pragma unroll
       for (int q = 0; q < 6; ++q) g[t][q] = out[q];
     }
@@ -408,11 +397,13 @@ template <typename S, typename R, bool PHYS>
 void launch_face_flux_kernel(const S* pool, const PatchDesc* patches, const FaceFluxOp* ops, int nops,
                              const double* b0, double gamma, int limiter, const FacePhysics& phys, double* reg,
                              cudaStream_t stream) {
+  const int splits = flux_splits(nops);
+  const int grid = int((int64_t(nops) * splits + kFluxWarps - 1) / kFluxWarps);
   switch (limiter) {
-    case 0: face_flux_ops_kernel<S, R, 0, PHYS><<<(nops + kFluxWarps - 1) / kFluxWarps, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    case 1: face_flux_ops_kernel<S, R, 1, PHYS><<<(nops + kFluxWarps - 1) / kFluxWarps, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    case 2: face_flux_ops_kernel<S, R, 2, PHYS><<<(nops + kFluxWarps - 1) / kFluxWarps, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    default: face_flux_ops_kernel<S, R, 3, PHYS><<<(nops + kFluxWarps - 1) / kFluxWarps, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    case 0: face_flux_ops_kernel<S, R, 0, PHYS><<<grid, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    case 1: face_flux_ops_kernel<S, R, 1, PHYS><<<grid, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    case 2: face_flux_ops_kernel<S, R, 2, PHYS><<<grid, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    default: face_flux_ops_kernel<S, R, 3, PHYS><<<grid, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
   }
 }
 
