@@ -32,8 +32,12 @@ __global__ void __launch_bounds__(kOpThreads) copy_ops_kernel(S* __restrict__ po
   copy_op_pairs(pool, patches, ops[blockIdx.x]);
 }
 
+// Blocks per SM the interpolation's registers are held to.
 template <typename S>
-__global__ void __launch_bounds__(kOpThreads) interp_ops_kernel(S* __restrict__ pool,
+constexpr int kInterpBlocks = sizeof(S) == 4 ? 16 : 12;
+
+template <typename S>
+__global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>) interp_ops_kernel(S* __restrict__ pool,
                                                                const PatchDesc* __restrict__ patches,
                                                                const InterpOp* __restrict__ ops) {
   interp_op(pool, patches, ops[blockIdx.x]);
@@ -44,7 +48,7 @@ __global__ void __launch_bounds__(kOpThreads) interp_ops_kernel(S* __restrict__ 
 // that another op of the launch writes or reads, as for interpolation ops trimmed to the
 // halo points no sibling covers (the copies read only their sources' computed points).
 template <typename S>
-__global__ void __launch_bounds__(kOpThreads) fill_ops_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
+__global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>) fill_ops_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
                                                              const InterpOp* __restrict__ interp, int ninterp,
                                                              const CopyOp* __restrict__ copies) {
   if (int(blockIdx.x) < ninterp)
