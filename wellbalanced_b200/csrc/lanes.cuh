@@ -34,10 +34,23 @@ __device__ __forceinline__ L1 sel(bool m, L1 a, L1 b) { return m ? a : b; }
 __device__ __forceinline__ L1 labs(L1 a) { return L1(fabsf(a.v)); }
 __device__ __forceinline__ L1 lmin(L1 a, L1 b) { return L1(fminf(a.v, b.v)); }
 __device__ __forceinline__ L1 lmax(L1 a, L1 b) { return L1(fmaxf(a.v, b.v)); }
+// three-operand min / max (one instruction of sm_100)
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ L1 lmin3(L1 a, L1 b, L1 c) { return L1(min3(a.v, b.v, c.v)); }
+__device__ __forceinline__ L1 lmax3(L1 a, L1 b, L1 c) { return L1(max3(a.v, b.v, c.v)); }
 __device__ __forceinline__ L1 lcopysign(L1 m, L1 s) { return L1(copysignf(m.v, s.v)); }
 // reciprocal and reciprocal square root from the special-function unit (~1 ulp)
-__device__ __forceinline__ L1 linv(L1 a) { return L1(__fdividef(1.0f, a.v)); }
-__device__ __forceinline__ L1 lrsqrt(L1 a) { return L1(rsqrtf(a.v)); }
+__device__ __forceinline__ L1 linv(L1 a) { return L1(rcp_ftz(a.v)); }
+__device__ __forceinline__ L1 lrsqrt(L1 a) { return L1(rsqrt_ftz(a.v)); }
 __device__ __forceinline__ bool any(bool m) { return m; }
 
 struct M2 {
@@ -83,9 +96,19 @@ __device__ __forceinline__ F2 sel(M2 m, F2 a, F2 b) { return F2(m.x ? a.v.x : b.
 __device__ __forceinline__ F2 labs(F2 a) { return F2(fabsf(a.v.x), fabsf(a.v.y)); }
 __device__ __forceinline__ F2 lmin(F2 a, F2 b) { return F2(fminf(a.v.x, b.v.x), fminf(a.v.y, b.v.y)); }
 __device__ __forceinline__ F2 lmax(F2 a, F2 b) { return F2(fmaxf(a.v.x, b.v.x), fmaxf(a.v.y, b.v.y)); }
+__device__ __forceinline__ F2 lmin3(F2 a, F2 b, F2 c) {
+  return F2(min3(a.v.x, b.v.x, c.v.x), min3(a.v.y, b.v.y, c.v.y));
+}
+__device__ __forceinline__ F2 lmax3(F2 a, F2 b, F2 c) {
+  return F2(max3(a.v.x, b.v.x, c.v.x), max3(a.v.y, b.v.y, c.v.y));
+}
 __device__ __forceinline__ F2 lcopysign(F2 m, F2 s) { return F2(copysignf(m.v.x, s.v.x), copysignf(m.v.y, s.v.y)); }
-__device__ __forceinline__ F2 linv(F2 a) { return F2(__fdividef(1.0f, a.v.x), __fdividef(1.0f, a.v.y)); }
-__device__ __forceinline__ F2 lrsqrt(F2 a) { return F2(rsqrtf(a.v.x), rsqrtf(a.v.y)); }
+__device__ __forceinline__ F2 linv(F2 a) { return F2(rcp_ftz(a.v.x), rcp_ftz(a.v.y)); }
+__device__ __forceinline__ F2 lrsqrt(F2 a) { return F2(rsqrt_ftz(a.v.x), rsqrt_ftz(a.v.y)); }
+// a b rounded on its own also where a sum follows: ptxas fuses a packed product into a packed
+// sum (the scalar intrinsics it leaves alone)
+__device__ __forceinline__ L1 lproduct(L1 a, L1 b) { return a * b; }
+__device__ __forceinline__ F2 lproduct(F2 a, F2 b) { return F2(__fmul_rn(a.v.x, b.v.x), __fmul_rn(a.v.y, b.v.y)); }
 // 0 - a (a negation for the packed type, kept identical in both lane types)
 template <typename V>
 __device__ __forceinline__ V lneg(V a) {

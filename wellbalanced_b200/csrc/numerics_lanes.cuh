@@ -14,27 +14,33 @@
 
 namespace wb {
 
+// What bounds these faces is instruction issue, and among the pipes the one that runs
+// selects, compares and min / max (half the rate of the multiply-adds): the forms below are
+// chosen for few of those, each with the bits of the plain selection. Per face: 57 fewer than
+// selecting every variant (limiter 14, square roots 6, first-order fallback 12, star states
+// 10, sign 3, region selection 12).
+
+// sqrt(x) as x rsqrt(x); x below the smallest normal (zero and negative discriminants) counts
+// as that, so the root of zero is 1e-19: far under the rounding of what it is added to.
 template <typename V>
-__device__ __forceinline__ V lsqrt(V x) {  // x > 0 ? sqrt(x) : 0, as x rsqrt(x)
-  return sel(x > V(0.0f), x * lrsqrt(x), V(0.0f));
+__device__ __forceinline__ V lsqrt(V x) {
+  const V y = lmax(x, V(kSmallestNormal));
+  return lproduct(y, lrsqrt(y));
 }
 
+// Half the limited slope of a cell from its backward (a) and forward (b) differences. minmod
+// and MC without a product or a sign test: the candidates nearest zero of one sign, the
+// other sign's clamp being zero (candidates of both signs clamp to zero twice).
 template <int LIM, typename V>
-__device__ __forceinline__ V limited_slope_l(V a, V b) {
-  if (LIM == 3) return V(0.5f) * (a + b);
-  const auto same = a * b > V(0.0f);
-  V slope;
-  if (LIM == 0) {
-    slope = sel(labs(a) < labs(b), a, b);
-  } else if (LIM == 1) {
-    const V sum = a + b;
-    slope = V(2.0f) * (a * b) * linv(sum);
-  } else {
-    const V central = V(0.5f) * (a + b);
-    const V bound = V(2.0f) * lmin(labs(a), labs(b));
-    slope = lcopysign(lmin(labs(central), bound), a);
+__device__ __forceinline__ V half_slope_l(V a, V b) {
+  if (LIM == 3) return V(0.25f) * (a + b);
+  if (LIM == 0) return V(0.5f) * (lmax(lmin(a, b), V(0.0f)) + lmin(lmax(a, b), V(0.0f)));
+  if (LIM == 1) {
+    const V product = a * b;
+    return sel(product > V(0.0f), product * linv(a + b), V(0.0f));
   }
-  return sel(same, slope, V(0.0f));
+  const V quarter = V(0.25f) * (a + b);
+  return lmax(lmin3(a, b, quarter), V(0.0f)) + lmin(lmax3(a, b, quarter), V(0.0f));
 }
 
 // Fast magnetosonic speed along the normal (the discriminant clipped at zero).
@@ -76,30 +82,32 @@ __device__ __forceinline__ V side_state_l(const V (&w)[7], V bn, V nbn, V inv_gm
   return pt;
 }
 
-// The wave speeds, S_M, p_T* and both sides' star density, tangential velocity and field.
+// The wave speeds, S_M, p_T* and both sides' star density, tangential velocity and field,
+// and 1 / (S - S_M).
 template <typename V>
 struct HlldFrontL {
   V sl, sr, ptl, ptr, sm, pts;
-  V rsl, vtl1, vtl2, btl1, btl2, den_l;
-  V rsr, vtr1, vtr2, btr1, btr2, den_r;
+  V rsl, vtl1, vtl2, btl1, btl2, inv_sl;
+  V rsr, vtr1, vtr2, btr1, btr2, inv_sr;
 };
 
-// Star tangential velocity and field of one side; `den` returns d (s - s_M) - B_n^2.
+// Star tangential velocity and field of one side; `den` returns d (s - s_M) - B_n^2. No test
+// for a vanishing denominator here: a face where it is small is redone in float64.
 template <typename V>
-__device__ __forceinline__ void star_tangential_l(const V (&w)[7], V bn, V bn2, V s, V d, V pt, V sm, V& rho_s,
-                                                  V& vt1, V& vt2, V& bt1, V& bt2, V& den) {
+__device__ __forceinline__ void star_tangential_l(const V (&w)[7], V bn, V bn2, V s, V d, V sm, V& rho_s, V& vt1,
+                                                  V& vt2, V& bt1, V& bt2, V& den, V& inv_ssm) {
   const V vn = w[1];
   const V ssm = s - sm;
-  rho_s = d * linv(ssm);
+  inv_ssm = linv(ssm);
+  rho_s = d * inv_ssm;
   den = fma(d, ssm, lneg(bn2));
-  const auto regular = labs(den) >= V(float(kDegenerate)) * (pt + bn2);
   const V inv_den = linv(den);
   const V scale = fma(d, s - vn, lneg(bn2)) * inv_den;
   const V shift = bn * (vn - sm) * inv_den;
-  vt1 = sel(regular, fma(shift, w[5], w[2]), w[2]);
-  vt2 = sel(regular, fma(shift, w[6], w[3]), w[3]);
-  bt1 = sel(regular, w[5] * scale, w[5]);
-  bt2 = sel(regular, w[6] * scale, w[6]);
+  vt1 = fma(shift, w[5], w[2]);
+  vt2 = fma(shift, w[6], w[3]);
+  bt1 = w[5] * scale;
+  bt2 = w[6] * scale;
 }
 
 // The front half of one face with its left and right sides in the two lanes of F2 (fast
@@ -128,15 +136,16 @@ __device__ __forceinline__ void hlld_front_lr(const float (&L)[7], const float (
   const L1 inv_dd = linv(dr - dl);
   o.sm = fma(dr, vr, fma(ndl, vl, o.ptl - o.ptr)) * inv_dd;
   o.pts = fma(dr, o.ptl, fma(ndl, o.ptr, dl * dr * (vr - vl))) * inv_dd;
-  F2 rho_s, vt1, vt2, bt1, bt2, den;
-  star_tangential_l<F2>(w, F2(bn), F2(bn2.v), s2, d2, pt2, F2(o.sm.v), rho_s, vt1, vt2, bt1, bt2, den);
+  F2 rho_s, vt1, vt2, bt1, bt2, den, inv_ssm;
+  star_tangential_l<F2>(w, F2(bn), F2(bn2.v), s2, d2, F2(o.sm.v), rho_s, vt1, vt2, bt1, bt2, den, inv_ssm);
   o.rsl = rho_s.v.x, o.rsr = rho_s.v.y;
   o.vtl1 = vt1.v.x, o.vtr1 = vt1.v.y;
   o.vtl2 = vt2.v.x, o.vtr2 = vt2.v.y;
   o.btl1 = bt1.v.x, o.btr1 = bt1.v.y;
   o.btl2 = bt2.v.x, o.btr2 = bt2.v.y;
-  o.den_l = den.v.x, o.den_r = den.v.y;
-  if (!any(labs(den) < F2(kNearDegenerate32) * (pt2 + F2(bn2.v)))) return;
+  o.inv_sl = inv_ssm.v.x, o.inv_sr = inv_ssm.v.y;
+  // (written so that a NaN or a zero denominator is redone too)
+  if (!any(!(labs(den) > F2(kNearDegenerate32) * (pt2 + F2(bn2.v))))) return;
   double Ld[7], Rd[7];
 #pragma unroll
   for (int c = 0; c < 7; ++c) {
@@ -148,21 +157,22 @@ __device__ __forceinline__ void hlld_front_lr(const float (&L)[7], const float (
   o.sl = float(d.sl), o.sr = float(d.sr), o.ptl = float(d.ptl), o.ptr = float(d.ptr);
   o.sm = float(d.sm), o.pts = float(d.pts);
   o.rsl = float(d.rsl), o.vtl1 = float(d.vtl1), o.vtl2 = float(d.vtl2);
-  o.btl1 = float(d.btl1), o.btl2 = float(d.btl2), o.den_l = float(d.den_l);
+  o.btl1 = float(d.btl1), o.btl2 = float(d.btl2), o.inv_sl = linv(o.sl - o.sm);
   o.rsr = float(d.rsr), o.vtr1 = float(d.vtr1), o.vtr2 = float(d.vtr2);
-  o.btr1 = float(d.btr1), o.btr2 = float(d.btr2), o.den_r = float(d.den_r);
+  o.btr1 = float(d.btr1), o.btr2 = float(d.btr2), o.inv_sr = linv(o.sr - o.sm);
 }
 
 // The back half of the HLLD flux from its front (straight-line code: the star / double-star
-// flux of the side of the contact the face lies on, selected at the end; as hlld_flux in
-// numerics.cuh).
+// flux of the side of the contact the face lies on; as hlld_flux in numerics.cuh).
 template <typename V>
 __device__ __forceinline__ void hlld_tail_l(const V (&L)[7], const V (&Rt)[7], V bn, V inv_gm1,
                                             const HlldFrontL<V>& fr, V (&F)[7]) {
   const V sm = fr.sm;
   const V sql = lsqrt(fr.rsl);
   const V sqr = lsqrt(fr.rsr);
-  const V sign = sel(bn > V(0.0f), V(1.0f), sel(bn < V(0.0f), V(-1.0f), V(0.0f)));
+  // the sign of B_n; where it is zero the Alfven waves lie on the contact, and the
+  // double-star state, its only use, is not taken
+  const V sign = lcopysign(V(1.0f), bn);
   const V inv_sum = linv(sql + sqr);
   const V vt2_1 = fma(sql, fr.vtl1, fma(sqr, fr.vtr1, (fr.btr1 - fr.btl1) * sign)) * inv_sum;
   const V vt2_2 = fma(sql, fr.vtl2, fma(sqr, fr.vtr2, (fr.btr2 - fr.btl2) * sign)) * inv_sum;
@@ -195,7 +205,7 @@ __device__ __forceinline__ void hlld_tail_l(const V (&L)[7], const V (&Rt)[7], V
   const V vb = fma(vn, bn, fma(w[2], w[5], w[3] * w[6]));
   const V vb_s = fma(sm, bn, fma(vt1, bt1, vt2 * bt2));
   const V energy_s =
-      fma(s - vn, u[4], fma(fr.pts, sm, fma(bn, vb - vb_s, lneg(pt) * vn))) * linv(s - sm);
+      fma(s - vn, u[4], fma(fr.pts, sm, fma(bn, vb - vb_s, lneg(pt) * vn))) * sel(left, fr.inv_sl, fr.inv_sr);
   V us[7], ud[7];
   us[0] = rho_s;
   us[1] = rho_s * sm;
@@ -209,12 +219,14 @@ __device__ __forceinline__ void hlld_tail_l(const V (&L)[7], const V (&Rt)[7], V
   ud[4] = fma(sense * sq * sign, vb_s - vb2, energy_s);
   ud[5] = bt2_1;
   ud[6] = bt2_2;
+  // f + S (U* - U) + S* (U** - U*), a wave speed the face lies outside of counting as zero
+  const V first = sel(supersonic, V(0.0f), s);
+  const V second = sel(!supersonic & twice, ss, V(0.0f));
 #pragma unroll
   for (int c = 0; c < 7; ++c) {
-    const V star = fma(s, us[c] - u[c], f[c]);
+    const V star = fma(first, us[c] - u[c], f[c]);
     // the double-star state differs from the star state in rows 2-6 only
-    const V twice_star = c < 2 ? star : fma(ss, ud[c] - us[c], star);
-    F[c] = sel(supersonic, f[c], sel(twice, twice_star, star));
+    F[c] = c < 2 ? star : fma(second, ud[c] - us[c], star);
   }
 }
 
@@ -243,6 +255,23 @@ __device__ __forceinline__ void hlld_flux(const float (&L)[7], const float (&Rt)
   from_lanes(f, F);
 }
 
+// The left / right states q +- h of a face from the two cells beside it and their half
+// slopes, (left, right) on the two lanes of F2. Where a density or pressure is not positive
+// the face falls back to first order: its slopes count with the factor `keep` = 0.
+__device__ __forceinline__ void face_states(const F2 (&q)[7], const F2 (&h)[7], float (&L)[7], float (&Rt)[7]) {
+  const F2 one(1.0f, -1.0f);
+  const F2 rho = fma(one, h[0], q[0]), p = fma(one, h[4], q[4]);
+  const float least = fminf(fminf(rho.v.x, rho.v.y), fminf(p.v.x, p.v.y));
+  const float keep = least > 0.0f ? 1.0f : 0.0f;
+  const F2 factor(keep, -keep);
+#pragma unroll
+  for (int c = 0; c < 7; ++c) {
+    const F2 lr = fma(factor, h[c], q[c]);
+    L[c] = lr.v.x;
+    Rt[c] = lr.v.y;
+  }
+}
+
 // One face's reconstruction with its left and right states in the two lanes of F2: the
 // two limited slopes of each component in one packed evaluation (lane x: the cell below the
 // face, lane y: the cell above), the states as one packed FMA. Lane by lane the same
@@ -250,55 +279,44 @@ __device__ __forceinline__ void hlld_flux(const float (&L)[7], const float (&Rt)
 template <int LIM>
 __device__ __forceinline__ void reconstruct(const float (&q0)[7], const float (&q1)[7], const float (&q2)[7],
                                             const float (&q3)[7], float (&L)[7], float (&Rt)[7]) {
-  const F2 half(0.5f, -0.5f);
+  F2 q[7], h[7];
 #pragma unroll
   for (int c = 0; c < 7; ++c) {
     const F2 a01(q0[c], q1[c]), a12(q1[c], q2[c]), a23(q2[c], q3[c]);
-    const F2 lr = fma(half, limited_slope_l<LIM>(a12 - a01, a23 - a12), a12);
-    L[c] = lr.v.x;
-    Rt[c] = lr.v.y;
+    q[c] = a12;
+    h[c] = half_slope_l<LIM>(a12 - a01, a23 - a12);
   }
-  const bool first_order = L[0] <= 0.0f || L[4] <= 0.0f || Rt[0] <= 0.0f || Rt[4] <= 0.0f;
-#pragma unroll
-  for (int c = 0; c < 7; ++c) {
-    L[c] = first_order ? q1[c] : L[c];
-    Rt[c] = first_order ? q2[c] : Rt[c];
-  }
+  face_states(q, h, L, Rt);
 }
 
-__device__ __forceinline__ void reconstruct_sloped(const float (&q1)[7], const float (&q2)[7], const float (&s1)[7],
-                                                   const float (&s2)[7], float (&L)[7], float (&Rt)[7]) {
-  const F2 half(0.5f, -0.5f);
+// The same from half slopes already formed (h1 of q1, h2 of q2).
+__device__ __forceinline__ void reconstruct_halves(const float (&q1)[7], const float (&q2)[7], const float (&h1)[7],
+                                                   const float (&h2)[7], float (&L)[7], float (&Rt)[7]) {
+  F2 q[7], h[7];
 #pragma unroll
   for (int c = 0; c < 7; ++c) {
-    const F2 lr = fma(half, F2(s1[c], s2[c]), F2(q1[c], q2[c]));
-    L[c] = lr.v.x;
-    Rt[c] = lr.v.y;
+    q[c] = F2(q1[c], q2[c]);
+    h[c] = F2(h1[c], h2[c]);
   }
-  const bool first_order = L[0] <= 0.0f || L[4] <= 0.0f || Rt[0] <= 0.0f || Rt[4] <= 0.0f;
-#pragma unroll
-  for (int c = 0; c < 7; ++c) {
-    L[c] = first_order ? q1[c] : L[c];
-    Rt[c] = first_order ? q2[c] : Rt[c];
-  }
+  face_states(q, h, L, Rt);
 }
 
-// Limited slopes of seven components from their backward (a) and forward (b) differences,
-// two components per packed evaluation (lane by lane as limited_slope_l<L1>).
+// Half slopes of seven components from their backward (a) and forward (b) differences, two
+// components per packed evaluation (lane by lane as half_slope_l<L1>).
 template <int LIM>
-__device__ __forceinline__ void limited_slopes7(const float (&a)[7], const float (&b)[7], float (&out)[7]) {
+__device__ __forceinline__ void half_slopes7(const float (&a)[7], const float (&b)[7], float (&out)[7]) {
 #pragma unroll
   for (int c = 0; c < 6; c += 2) {
-    const F2 s = limited_slope_l<LIM>(F2(a[c], a[c + 1]), F2(b[c], b[c + 1]));
+    const F2 s = half_slope_l<LIM>(F2(a[c], a[c + 1]), F2(b[c], b[c + 1]));
     out[c] = s.v.x;
     out[c + 1] = s.v.y;
   }
-  out[6] = limited_slope_l<LIM>(L1(a[6]), L1(b[6])).v;
+  out[6] = half_slope_l<LIM>(L1(a[6]), L1(b[6])).v;
 }
 
 template <int LIM>
 __device__ __forceinline__ float limited_slope(float a, float b) {
-  return limited_slope_l<LIM>(L1(a), L1(b)).v;
+  return 2.0f * half_slope_l<LIM>(L1(a), L1(b)).v;
 }
 
 }  // namespace wb

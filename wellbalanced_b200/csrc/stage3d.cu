@@ -354,7 +354,8 @@ __global__ void __launch_bounds__(threads3d<TY, TZ>(), (Occupancy3D<R, PHYS, TY,
         q1[cc] = loaded ? Pc[xrow[cc] * NR + col_r] : R(1);
         q2[cc] = Pn[xrow[cc] * NR + col_r];
       }
-      // the slope of plane p, kept for face p + 1: each cell's x-slope is formed once
+      // the slope (float32: its half) of plane p, kept for face p + 1: each cell's x-slope is
+      // formed once
       R now[7];
       if constexpr (std::is_same<R, float>::value) {
         float back[7], fwd[7];
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(threads3d<TY, TZ>(), (Occupancy3D<R, PHYS, TY,
           back[cc] = q1[cc] - qm[cc];
           fwd[cc] = q2[cc] - q1[cc];
         }
-        limited_slopes7<LIM>(back, fwd, now);
+        half_slopes7<LIM>(back, fwd, now);
       } else {
 #pragma unroll
         for (int cc = 0; cc < 7; ++cc) now[cc] = limited_slope<LIM>(q1[cc] - qm[cc], q2[cc] - q1[cc]);
@@ -371,7 +372,10 @@ __global__ void __launch_bounds__(threads3d<TY, TZ>(), (Occupancy3D<R, PHYS, TY,
       const R* Bp = sBn + (PHYS ? face_slot<PHYS>(p) : ((p + 4) & 1)) * 3 * NR;
       if (p >= x0) {
         R L[7], Rt[7], F[7];
-        reconstruct_sloped(qm, q1, slope, now, L, Rt);
+        if constexpr (std::is_same<R, float>::value)
+          reconstruct_halves(qm, q1, slope, now, L, Rt);
+        else
+          reconstruct_sloped(qm, q1, slope, now, L, Rt);
         hlld_flux(L, Rt, Bp[col_r], gamma, inv_gm1, F);
         if (PHYS && a.eta != 0.0 && tid < NCORE) {
           // eta (J_y B_z - J_z B_y) on the x-face: J of its two y- and two z-edges, B of
