@@ -165,6 +165,18 @@ int wb_finalize_dt(const unsigned long long* keys, int ninstances, double cfl, d
                    double gamma, const double* inv_dx2_sum, double* time, const double* end, double* dt,
                    int advance, void* stream);
 
+/* wb_rate and wb_finalize_dt in one launch (with level_keys, inv_dx2_levels and nlevels:
+ * wb_rate_levels and wb_finalize_dt_levels; level_keys NULL: without levels). The same keys,
+ * level_keys and dt. scratch: 1 + 2 ninstances (+ ninstances nlevels) 64-bit words, a ticket
+ * (0) and the identities of the keys (per instance 0x8000000000000000, 0xfff0000000000000;
+ * per level 0xfff0000000000000); every launch leaves it so. Launches that share a scratch
+ * must not overlap. */
+int wb_stable_dt(int precision, int ndim, const void* state, const void* patches, const int* chunk_patch,
+                 const int* chunk_start, int nchunks, double b0x, double b0y, double b0z, double gamma,
+                 unsigned long long* keys, int ninstances, unsigned long long* level_keys, int nlevels, double cfl,
+                 double eta, double kappa, const double* inv_dx2_sum, const double* inv_dx2_levels, double* time,
+                 const double* end, double* dt, int advance, unsigned long long* scratch, void* stream);
+
 /* wb_rate that also reduces the smallest density of every (instance, level):
  * level_keys[instance * nlevels + level] (order-preserving keys, nlevels * ninstances).
  * With wb_finalize_dt_levels it takes the diffusion limit level by level, each level's

@@ -47,6 +47,8 @@ SIGNATURES = {
     "wb_rate": [c_int, c_int, c_dp, c_dp, c_int, c_dp, c_dp, c_int, c_double, c_double, c_double, c_double, c_dp,
                 c_int, c_dp],
     "wb_finalize_dt": [c_dp, c_int, c_double, c_double, c_double, c_double, c_dp, c_dp, c_dp, c_dp, c_int, c_dp],
+    "wb_stable_dt": [c_int, c_int, c_dp, c_dp, c_dp, c_dp, c_int, c_double, c_double, c_double, c_double, c_dp, c_int,
+                     c_dp, c_int, c_double, c_double, c_double, c_dp, c_dp, c_dp, c_dp, c_dp, c_int, c_dp, c_dp],
     "wb_rate_levels": [c_int, c_int, c_dp, c_dp, c_int, c_dp, c_dp, c_int, c_double, c_double, c_double, c_double,
                        c_dp, c_int, c_dp, c_int, c_dp],
     "wb_finalize_dt_levels": [c_dp, c_int, c_double, c_double, c_double, c_double, c_dp, c_dp, c_int, c_dp, c_dp,

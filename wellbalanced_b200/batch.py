@@ -128,8 +128,7 @@ class Batch:
         eng = self.engine
         groups = eng.layout.groups
         with eng.launching():
-            eng.rate()
-            eng.finalize_dt(self.cfl, advance=True)
+            eng.stable_dt(self.cfl, advance=True)
             eng.heun_step(groups[1:], groups)
 
     def capture(self):

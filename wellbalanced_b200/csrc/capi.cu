@@ -407,6 +407,38 @@ int wb_finalize_dt_levels(const unsigned long long* keys, int ninstances, double
                             as_stream(stream), level_keys, inv_dx2_levels, nlevels);
 }
 
+int wb_stable_dt(int precision, int ndim, const void* state, const void* patches, const int* chunk_patch,
+                 const int* chunk_start, int nchunks, double b0x, double b0y, double b0z, double gamma,
+                 unsigned long long* keys, int ninstances, unsigned long long* level_keys, int nlevels, double cfl,
+                 double eta, double kappa, const double* inv_dx2_sum, const double* inv_dx2_levels, double* time,
+                 const double* end, double* dt, int advance, unsigned long long* scratch, void* stream) {
+  set_error("");
+  if (!precision_ok(precision, "stable_dt") || !ptrs_ok({state, patches, keys, inv_dx2_sum, dt, scratch}, "stable_dt"))
+    return kBadArgument;
+  if ((ndim != 2 && ndim != 3) || ninstances <= 0 || nchunks < 0 || (nchunks > 0 && (!chunk_patch || !chunk_start)) ||
+      (level_keys && (nlevels <= 0 || !inv_dx2_levels))) {
+    set_error("stable_dt: bad ndim / ninstances / levels / work list");
+    return kBadArgument;
+  }
+  if (level_keys && int64_t(ninstances) * nlevels >= (int64_t(1) << 31)) {
+    set_error("stable_dt: %d instances x %d levels exceed 2^31 keys", ninstances, nlevels);
+    return kTooLarge;
+  }
+  if ((end || advance) && !time) {
+    set_error("stable_dt: time is required with end or advance");
+    return kBadArgument;
+  }
+  const double b0[3] = {b0x, b0y, b0z};
+  const PatchDesc* rows = static_cast<const PatchDesc*>(patches);
+  if (precision == 32)
+    return launch_stable_dt<float>(static_cast<const float*>(state), rows, ndim, chunk_patch, chunk_start, nchunks, b0,
+                                   gamma, keys, ninstances, level_keys, nlevels, cfl, eta, kappa, inv_dx2_sum,
+                                   inv_dx2_levels, time, end, dt, advance, scratch, as_stream(stream));
+  return launch_stable_dt<double>(static_cast<const double*>(state), rows, ndim, chunk_patch, chunk_start, nchunks, b0,
+                                  gamma, keys, ninstances, level_keys, nlevels, cfl, eta, kappa, inv_dx2_sum,
+                                  inv_dx2_levels, time, end, dt, advance, scratch, as_stream(stream));
+}
+
 int wb_copy_ops(int precision, void* pool, const void* patches, const void* ops, int nops, void* stream) {
   set_error("");
   if (!precision_ok(precision, "copy_ops") || !ptrs_ok({pool, patches}, "copy_ops") || (nops > 0 && !ops))

@@ -97,4 +97,122 @@ int launch_finalize_dt(const unsigned long long* keys, int ninstances, double cf
   return check_launch("finalize_dt");
 }
 
+// The stable step in one launch: `parts` blocks share each 2048-cell chunk of the work list;
+// a block reduces its cells, takes the maximum and minimum to the scratch keys (an atomic only
+// where it would change the key), and the last block to finish turns the keys into every
+// instance's dt, hands them on in `keys` / `level_keys` and puts the scratch back to the
+// identities for the next launch. Three launches (keys, rate, dt) and 8 serial rounds a block
+// before; small grids, whose few chunks left most SMs idle, take 8 blocks a chunk.
+struct StableDt {
+  double cfl, eta, kappa, gamma;
+  const double *inv_dx2_sum, *inv_dx2_levels;
+  double* time;
+  const double* end;
+  double* dt;
+  int advance;
+  unsigned long long *keys, *level_keys;  // the results (level_keys nullable)
+};
+
+// (float32: 32 registers, 64 warps an SM, as the rate kernel alone)
+template <typename S, int NDIM>
+__global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4) stable_dt_kernel(const S* __restrict__ pool, const PatchDesc* patches,
+                                                                 const int* chunk_patch, const int* chunk_start,
+                                                                 int nchunks, int parts, double b0x, double b0y,
+                                                                 double b0z, const RateSlots scratch,
+                                                                 unsigned long long* ticket, const StableDt a) {
+  __shared__ double s_largest[kRateThreads / 32], s_smallest[kRateThreads / 32];
+  __shared__ bool s_last;
+  const int chunk = int(blockIdx.x) / parts, part = int(blockIdx.x) - chunk * parts;
+  if (chunk < nchunks) {
+    const PatchDesc P = patches[chunk_patch[chunk]];
+    unsigned long long *keys, *level_min;
+    if (rate_slot(P, scratch, &keys, &level_min)) {  // uniform over the block
+      const int rounds = int(kRateChunk / kRateThreads) / parts;
+      const unsigned begin = unsigned(chunk_start[chunk]) + unsigned(part * rounds * kRateThreads);
+      S largest = S(0), smallest = S(INFINITY);
+      if (NDIM == 2)
+        rate_cells2d<S, kRateThreads>(pool + P.off, P, begin, rounds, b0x, b0y, a.gamma, largest, smallest);
+      else
+        rate_cells3d<S, kRateThreads>(pool + P.off, P, begin, rounds, b0x, b0y, b0z, a.gamma, largest, smallest);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        largest = rmax(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+        smallest = rmin(smallest, __shfl_xor_sync(0xffffffffu, smallest, o));
+      }
+      if ((threadIdx.x & 31) == 0) {
+        s_largest[threadIdx.x >> 5] = double(largest);
+        s_smallest[threadIdx.x >> 5] = double(smallest);
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double top = s_largest[0], low = s_smallest[0];
+#pragma unroll
+        for (int w = 1; w < kRateThreads / 32; ++w) {
+          top = fmax(top, s_largest[w]);
+          low = fmin(low, s_smallest[w]);
+        }
+        const unsigned long long kt = double_to_key(top), kl = double_to_key(low);
+        if (kt > *static_cast<volatile unsigned long long*>(keys)) atomicMax(keys, kt);
+        if (kl < *static_cast<volatile unsigned long long*>(keys + 1)) atomicMin(keys + 1, kl);
+        if (level_min && kl < *static_cast<volatile unsigned long long*>(level_min)) atomicMin(level_min, kl);
+      }
+    }
+  }
+  if (threadIdx.x == 0) {
+    __threadfence();  // the block's keys before its ticket
+    s_last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();  // the other blocks' keys after their tickets
+  const int n = scratch.ninstances, nlevels = scratch.nlevels;
+  for (int i = threadIdx.x; i < n; i += kRateThreads) {
+    a.keys[2 * i] = __ldcg(scratch.keys + 2 * i);
+    a.keys[2 * i + 1] = __ldcg(scratch.keys + 2 * i + 1);
+    scratch.keys[2 * i] = double_to_key(0.0);
+    scratch.keys[2 * i + 1] = rate_min_identity();
+    if (scratch.level_keys)
+      for (int l = 0; l < nlevels; ++l) {
+        a.level_keys[i * nlevels + l] = __ldcg(scratch.level_keys + i * nlevels + l);
+        scratch.level_keys[i * nlevels + l] = rate_min_identity();
+      }
+    finalize_dt_one(i, a.keys, a.cfl, a.eta, a.kappa, a.gamma, a.inv_dx2_sum, a.level_keys, a.inv_dx2_levels, nlevels,
+                    a.time, a.end, a.dt, a.advance);
+  }
+  if (threadIdx.x == 0) *ticket = 0;
+}
+
+// scratch: 1 + 2 ninstances (+ ninstances nlevels) words: the ticket (0), then (key(0),
+// key(+inf)) per instance and key(+inf) per level, as every launch leaves them.
+template <typename S>
+int launch_stable_dt(const S* state, const PatchDesc* patches, int ndim, const int* chunk_patch,
+                     const int* chunk_start, int nchunks, const double* b0, double gamma, unsigned long long* keys,
+                     int ninstances, unsigned long long* level_keys, int nlevels, double cfl, double eta, double kappa,
+                     const double* inv_dx2_sum, const double* inv_dx2_levels, double* time, const double* end,
+                     double* dt, int advance, unsigned long long* scratch, cudaStream_t stream) {
+  const RateSlots slots{scratch + 1, ninstances, level_keys ? scratch + 1 + 2 * ninstances : nullptr, nlevels, nullptr};
+  const StableDt a{cfl, eta, kappa, gamma, inv_dx2_sum, inv_dx2_levels, time, end, dt, advance, keys, level_keys};
+  // up to 8 blocks a chunk while they make at most 4 blocks an SM: a block costs ~3 us besides
+  // its cells (work-list look-up, reduction, ticket), which more rounds carry better
+  int parts = 8;
+  while (parts > 1 && int64_t(nchunks) * parts > 148 * 4) parts /= 2;
+  const int grid = max(nchunks * parts, 1);
+  if (ndim == 2)
+    stable_dt_kernel<S, 2><<<grid, kRateThreads, 0, stream>>>(state, patches, chunk_patch, chunk_start, nchunks, parts,
+                                                             b0[0], b0[1], b0[2], slots, scratch, a);
+  else
+    stable_dt_kernel<S, 3><<<grid, kRateThreads, 0, stream>>>(state, patches, chunk_patch, chunk_start, nchunks, parts,
+                                                             b0[0], b0[1], b0[2], slots, scratch, a);
+  return check_launch("stable_dt");
+}
+
+template int launch_stable_dt<float>(const float*, const PatchDesc*, int, const int*, const int*, int, const double*,
+                                     double, unsigned long long*, int, unsigned long long*, int, double, double,
+                                     double, const double*, const double*, double*, const double*, double*, int,
+                                     unsigned long long*, cudaStream_t);
+template int launch_stable_dt<double>(const double*, const PatchDesc*, int, const int*, const int*, int, const double*,
+                                      double, unsigned long long*, int, unsigned long long*, int, double, double,
+                                      double, const double*, const double*, double*, const double*, double*, int,
+                                      unsigned long long*, cudaStream_t);
+
 }  // namespace wb

@@ -40,8 +40,156 @@ __device__ __forceinline__ bool rate_slot(const PatchDesc& P, const RateSlots& r
   return true;
 }
 
+// The rate's arithmetic with every rounding written out, so that each kernel that forms a
+// cell's rate (one launch or several, any unrolling) gets the same bits: left to the
+// compiler, the choice which product of a sum to fuse differed between instantiations in
+// one cell of twenty.
+template <typename S>
+struct RateMath;
+
+template <>
+struct RateMath<float> {
+  static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+  static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+  static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+  static __device__ __forceinline__ float div(float a, float, float inv_b) { return __fmul_rn(a, inv_b); }
+  // a / b + c and a / h - b / k
+  static __device__ __forceinline__ float div_plus(float a, float, float inv_b, float c) { return __fmaf_rn(a, inv_b, c); }
+  static __device__ __forceinline__ float curl(float a, float, float ih, float b, float, float ik) {
+    return __fmaf_rn(a, ih, -__fmul_rn(b, ik));
+  }
+  static __device__ __forceinline__ float sqrt(float x) {
+    return x >= kSmallestNormal ? __fmul_rn(x, rsqrt_ftz(x)) : 0.0f;
+  }
+};
+
+template <>
+struct RateMath<double> {
+  static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+  static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+  static __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+  static __device__ __forceinline__ double div(double a, double b, double inv_b) { return Math<double>::div(a, b, inv_b); }
+  static __device__ __forceinline__ double div_plus(double a, double b, double inv_b, double c) {
+    return __dadd_rn(div(a, b, inv_b), c);
+  }
+  static __device__ __forceinline__ double curl(double a, double h, double ih, double b, double k, double ik) {
+    return __dadd_rn(div(a, h, ih), -div(b, k, ik));
+  }
+  static __device__ __forceinline__ double sqrt(double x) { return x > 0.0 ? ::sqrt(x) : 0.0; }
+};
+
+// Fast magnetosonic speed from a2 = gamma p / rho, the normal field and the field squared.
+template <typename S, int NDIM>
+__device__ __forceinline__ S rate_speed(S a2, S bn, S field2, S rho, S inv_rho) {
+  using Q = RateMath<S>;
+  const S s = Q::div_plus(field2, rho, inv_rho, a2);
+  const S y = Q::mul(Q::mul(Q::mul(S(4), a2), bn), bn);
+  const S disc = NDIM == 2 ? Q::div_plus(-y, rho, inv_rho, Q::mul(s, s)) : Q::fma(s, s, -Q::div(y, rho, inv_rho));
+  const S root = disc > S(0) ? Q::sqrt(disc) : S(0);
+  return Q::sqrt(Q::mul(S(0.5), Q::add(s, root)));
+}
+
+// (gamma - 1) (E - rho v^2 / 2 - B^2 / 2)
+template <typename S>
+__device__ __forceinline__ S rate_pressure(S gm1, S e, S rho, S u, S v, S w, S field2) {
+  using Q = RateMath<S>;
+  const S v2 = Q::fma(w, w, Q::fma(u, u, Q::mul(v, v)));
+  const S rest = Q::fma(-Q::mul(S(0.5), rho), v2, e);
+  return Q::mul(gm1, Q::add(rest, -Q::mul(S(0.5), field2)));
+}
+
+// Largest signal rate and smallest density of the cells begin + thread, begin + thread + NT,
+// ... (`rounds` of them, those inside the patch). Issue and latency bound (~200 instructions
+// a float32 3D cell against 32 bytes); unrolling by two raises the registers and loses warps.
+// 2D:
+template <typename S, int NT>
+__device__ __forceinline__ void rate_cells2d(const S* __restrict__ src, const PatchDesc& P, unsigned begin, int rounds,
+                                             double b0x, double b0y, double gamma, S& largest, S& smallest) {
+  const int64_t pitch = P.pitch0, fs = P.fstride;
+  using M = Math<S>;
+  using Q = RateMath<S>;
+  const S dx = S(P.dx[0]), dy = S(P.dx[1]);
+  const S idx = M::inv(dx), idy = M::inv(dy);
+  const S g = S(gamma), gm1 = g - S(1), bx0 = S(b0x), by0 = S(b0y);
+  // work-list indices are 32-bit (chunk_start is int): 32-bit index arithmetic
+  const int ny = P.n[1];
+  const unsigned total = unsigned(P.n[0]) * unsigned(ny);
+#pragma unroll 1
+  for (int s = 0; s < rounds; ++s) {
+    const unsigned t = begin + unsigned(s) * NT + threadIdx.x;
+    if (t >= total) continue;
+    const unsigned row = t / unsigned(ny);
+    const int i = int(row) + kHalo, j = int(t - row * unsigned(ny)) + kHalo;
+    const int64_t c = int64_t(i) * pitch + j;
+    const S* A = src + 6 * fs;
+    const S a00 = A[c], a01 = A[c + 1], a10 = A[c + pitch], a11 = A[c + pitch + 1];
+    const S r = src[c];
+    const S ir = M::inv(r);
+    const S u = Q::div(src[fs + c], r, ir), v = Q::div(src[2 * fs + c], r, ir), w = Q::div(src[3 * fs + c], r, ir);
+    const S bz = src[5 * fs + c], e = src[4 * fs + c];
+    const S bx = Q::mul(S(0.5), Q::add(Q::div_plus(a01 - a00, dy, idy, bx0), Q::div_plus(a11 - a10, dy, idy, bx0)));
+    const S by = Q::mul(S(0.5), Q::add(Q::div_plus(a00 - a10, dx, idx, by0), Q::div_plus(a01 - a11, dx, idx, by0)));
+    const S b2 = Q::fma(bz, bz, Q::fma(bx, bx, Q::mul(by, by)));
+    const S p = rate_pressure(gm1, e, r, u, v, w, b2);
+    const S a2 = Q::div(Q::mul(g, p), r, ir);
+    const S cx = Q::add(rabs(u), rate_speed<S, 2>(a2, bx, b2, r, ir));
+    const S cy = Q::add(rabs(v), rate_speed<S, 2>(a2, by, b2, r, ir));
+    largest = rmax(largest, Q::div_plus(cx, dx, idx, Q::div(cy, dy, idy)));
+    smallest = rmin(smallest, r);
+  }
+}
+
+// 3D:
+template <typename S, int NT>
+__device__ __forceinline__ void rate_cells3d(const S* __restrict__ src, const PatchDesc& P, unsigned begin, int rounds,
+                                             double b0x, double b0y, double b0z, double gamma, S& largest, S& smallest) {
+  const int64_t p0 = P.pitch0, p1 = P.pitch1, fs = P.fstride;
+  using M = Math<S>;
+  using Q = RateMath<S>;
+  const S dx = S(P.dx[0]), dy = S(P.dx[1]), dz = S(P.dx[2]);
+  const S idx = M::inv(dx), idy = M::inv(dy), idz = M::inv(dz);
+  const S g = S(gamma), gm1 = g - S(1);
+  // work-list indices are 32-bit (chunk_start is int): 32-bit index arithmetic
+  const int ny = P.n[1], nz = P.n[2];
+  const unsigned total = unsigned(P.n[0]) * unsigned(ny) * unsigned(nz);
+#pragma unroll 1
+  for (int s = 0; s < rounds; ++s) {
+    const unsigned t = begin + unsigned(s) * NT + threadIdx.x;
+    if (t >= total) continue;
+    const unsigned line = t / unsigned(nz);
+    const unsigned plane = line / unsigned(ny);
+    const int i = int(plane) + kHalo;
+    const int j = int(line - plane * unsigned(ny)) + kHalo;
+    const int k = int(t - line * unsigned(nz)) + kHalo;
+    const int64_t o = int64_t(i) * p0 + int64_t(j) * p1 + k;
+    const S* Ax = src + 5 * fs;
+    const S* Ay = src + 6 * fs;
+    const S* Az = src + 7 * fs;
+    auto fx = [&](int64_t c) { return Q::add(Q::curl(Az[c + p1] - Az[c], dy, idy, Ay[c + 1] - Ay[c], dz, idz), S(b0x)); };
+    auto fy = [&](int64_t c) { return Q::add(Q::curl(Ax[c + 1] - Ax[c], dz, idz, Az[c + p0] - Az[c], dx, idx), S(b0y)); };
+    auto fz = [&](int64_t c) { return Q::add(Q::curl(Ay[c + p0] - Ay[c], dx, idx, Ax[c + p1] - Ax[c], dy, idy), S(b0z)); };
+    const S bx = Q::mul(S(0.5), Q::add(fx(o), fx(o + p0)));
+    const S by = Q::mul(S(0.5), Q::add(fy(o), fy(o + p1)));
+    const S bz = Q::mul(S(0.5), Q::add(fz(o), fz(o + 1)));
+    const S r = src[o];
+    const S ir = M::inv(r);
+    const S u = Q::div(src[fs + o], r, ir), v = Q::div(src[2 * fs + o], r, ir), w = Q::div(src[3 * fs + o], r, ir);
+    const S x2 = Q::mul(bx, bx), y2 = Q::mul(by, by), z2 = Q::mul(bz, bz);
+    const S xy = Q::add(x2, y2), yz = Q::add(y2, z2), zx = Q::add(z2, x2);
+    const S p = rate_pressure(gm1, src[4 * fs + o], r, u, v, w, Q::add(xy, z2));
+    const S a2 = Q::div(Q::mul(g, p), r, ir);
+    const S cx = Q::add(rabs(u), rate_speed<S, 3>(a2, bx, Q::add(xy, z2), r, ir));
+    const S cy = Q::add(rabs(v), rate_speed<S, 3>(a2, by, Q::add(yz, x2), r, ir));
+    const S cz = Q::add(rabs(w), rate_speed<S, 3>(a2, bz, Q::add(zx, y2), r, ir));
+    largest = rmax(largest, Q::div_plus(cz, dz, idz, Q::div_plus(cx, dx, idx, Q::div(cy, dy, idy))));
+    smallest = rmin(smallest, r);
+  }
+}
+
 // The cells of one chunk (kRateChunk cells of patch pi from `chunk_start`) over the NT
-// threads of a block, reduced into the chunk's slots. 2D:
+// threads of a block, reduced into the chunk's slots: the max / min in the state's type
+// (exact: the max of the float rates converts to the max of their double images), converted
+// once for the block reduction. 2D:
 template <typename S, int NT>
 __device__ __forceinline__ void rate_chunk2d(const S* __restrict__ pool, const PatchDesc* patches, int pi,
                                              int chunk_start, double b0x, double b0y, double gamma,
@@ -49,37 +197,8 @@ __device__ __forceinline__ void rate_chunk2d(const S* __restrict__ pool, const P
   const PatchDesc P = patches[pi];
   unsigned long long *keys, *level_min;
   if (!rate_slot(P, slots, &keys, &level_min)) return;  // uniform over the block
-  const int nx = P.n[0], ny = P.n[1];
-  const S* src = pool + P.off;
-  const int64_t pitch = P.pitch0, fs = P.fstride;
-  using M = Math<S>;
-  const S dx = S(P.dx[0]), dy = S(P.dx[1]);
-  const S idx = M::inv(dx), idy = M::inv(dy);
-  const S g = S(gamma), bx0 = S(b0x), by0 = S(b0y);
-  S largest = S(0), smallest = S(INFINITY);  // converted once, exactly (as in 3D)
-  // work-list indices are 32-bit (chunk_start is int): 32-bit index arithmetic
-  const unsigned total = unsigned(nx) * unsigned(ny);
-  const unsigned start = unsigned(chunk_start);
-#pragma unroll 2
-  for (int s = 0; s < int(kRateChunk / NT); ++s) {
-    const unsigned t = start + unsigned(s) * NT + threadIdx.x;
-    if (t >= total) continue;
-    const unsigned row = t / unsigned(ny);
-    const int i = int(row) + kHalo, j = int(t - row * unsigned(ny)) + kHalo;
-    const int64_t c = int64_t(i) * pitch + j;
-    const S* A = src + 6 * fs;
-    const S r = src[c];
-    const S ir = M::inv(r);
-    const S u = M::div(src[fs + c], r, ir), v = M::div(src[2 * fs + c], r, ir), w = M::div(src[3 * fs + c], r, ir);
-    const S bx = S(0.5) * (M::div(A[c + 1] - A[c], dy, idy) + bx0 + (M::div(A[c + pitch + 1] - A[c + pitch], dy, idy) + bx0));
-    const S by = S(0.5) * (-M::div(A[c + pitch] - A[c], dx, idx) + by0 + (-M::div(A[c + pitch + 1] - A[c + 1], dx, idx) + by0));
-    const S bz = src[5 * fs + c];
-    const S p = (g - S(1)) * (src[4 * fs + c] - S(0.5) * r * (u * u + v * v + w * w) - S(0.5) * (bx * bx + by * by + bz * bz));
-    const S rate = M::div(rabs(u) + fast_speed(r, p, bx, by, bz, g), dx, idx) +
-                   M::div(rabs(v) + fast_speed(r, p, by, bx, bz, g), dy, idy);
-    largest = rmax(largest, rate);
-    smallest = rmin(smallest, r);
-  }
+  S largest = S(0), smallest = S(INFINITY);
+  rate_cells2d<S, NT>(pool + P.off, P, unsigned(chunk_start), int(kRateChunk / NT), b0x, b0y, gamma, largest, smallest);
   block_reduce_keys(double(largest), double(smallest), keys, level_min);
 }
 
@@ -91,49 +210,9 @@ __device__ __forceinline__ void rate_chunk3d(const S* __restrict__ pool, const P
   const PatchDesc P = patches[pi];
   unsigned long long *keys, *level_min;
   if (!rate_slot(P, slots, &keys, &level_min)) return;  // uniform over the block
-  const int nx = P.n[0], ny = P.n[1], nz = P.n[2];
-  const S* src = pool + P.off;
-  const int64_t p0 = P.pitch0, p1 = P.pitch1, fs = P.fstride;
-  using M = Math<S>;
-  const S dx = S(P.dx[0]), dy = S(P.dx[1]), dz = S(P.dx[2]);
-  const S idx = M::inv(dx), idy = M::inv(dy), idz = M::inv(dz);
-  const S g = S(gamma);
-  // the max / min in the state's type (exact: the max of the float rates converts to the
-  // max of their double images), converted once for the block reduction
   S largest = S(0), smallest = S(INFINITY);
-  // work-list indices are 32-bit (chunk_start is int): 32-bit index arithmetic
-  const unsigned total = unsigned(nx) * unsigned(ny) * unsigned(nz);
-  const unsigned start = unsigned(chunk_start);
-#pragma unroll 2
-  for (int s = 0; s < int(kRateChunk / NT); ++s) {
-    const unsigned t = start + unsigned(s) * NT + threadIdx.x;
-    if (t >= total) continue;
-    const unsigned line = t / unsigned(nz);
-    const unsigned plane = line / unsigned(ny);
-    const int i = int(plane) + kHalo;
-    const int j = int(line - plane * unsigned(ny)) + kHalo;
-    const int k = int(t - line * unsigned(nz)) + kHalo;
-    const int64_t o = int64_t(i) * p0 + int64_t(j) * p1 + k;
-    const S* Ax = src + 5 * fs;
-    const S* Ay = src + 6 * fs;
-    const S* Az = src + 7 * fs;
-    const S bxl = M::div(Az[o + p1] - Az[o], dy, idy) - M::div(Ay[o + 1] - Ay[o], dz, idz) + S(b0x);
-    const S bxh = M::div(Az[o + p0 + p1] - Az[o + p0], dy, idy) - M::div(Ay[o + p0 + 1] - Ay[o + p0], dz, idz) + S(b0x);
-    const S byl = M::div(Ax[o + 1] - Ax[o], dz, idz) - M::div(Az[o + p0] - Az[o], dx, idx) + S(b0y);
-    const S byh = M::div(Ax[o + p1 + 1] - Ax[o + p1], dz, idz) - M::div(Az[o + p1 + p0] - Az[o + p1], dx, idx) + S(b0y);
-    const S bzl = M::div(Ay[o + p0] - Ay[o], dx, idx) - M::div(Ax[o + p1] - Ax[o], dy, idy) + S(b0z);
-    const S bzh = M::div(Ay[o + p0 + 1] - Ay[o + 1], dx, idx) - M::div(Ax[o + p1 + 1] - Ax[o + 1], dy, idy) + S(b0z);
-    const S bx = S(0.5) * (bxl + bxh), by = S(0.5) * (byl + byh), bz = S(0.5) * (bzl + bzh);
-    const S r = src[o];
-    const S ir = M::inv(r);
-    const S u = M::div(src[fs + o], r, ir), v = M::div(src[2 * fs + o], r, ir), w = M::div(src[3 * fs + o], r, ir);
-    const S p = (g - S(1)) * (src[4 * fs + o] - S(0.5) * r * (u * u + v * v + w * w) - S(0.5) * (bx * bx + by * by + bz * bz));
-    const S rate = M::div(rabs(u) + fast_speed(r, p, bx, by, bz, g), dx, idx) +
-                   M::div(rabs(v) + fast_speed(r, p, by, bz, bx, g), dy, idy) +
-                   M::div(rabs(w) + fast_speed(r, p, bz, bx, by, g), dz, idz);
-    largest = rmax(largest, rate);
-    smallest = rmin(smallest, r);
-  }
+  rate_cells3d<S, NT>(pool + P.off, P, unsigned(chunk_start), int(kRateChunk / NT), b0x, b0y, b0z, gamma, largest,
+                      smallest);
   block_reduce_keys(double(largest), double(smallest), keys, level_min);
 }
 

@@ -63,6 +63,14 @@ int launch_rate_chunks(const S* state, const PatchDesc* patches, int npatches, i
                        unsigned long long* keys, int ninstances, cudaStream_t stream,
                        unsigned long long* level_keys = nullptr, int nlevels = 0, unsigned* error = nullptr);
 
+// The rate and dt of the two functions around this one in a single launch (rate.cu).
+template <typename S>
+int launch_stable_dt(const S* state, const PatchDesc* patches, int ndim, const int* chunk_patch,
+                     const int* chunk_start, int nchunks, const double* b0, double gamma, unsigned long long* keys,
+                     int ninstances, unsigned long long* level_keys, int nlevels, double cfl, double eta, double kappa,
+                     const double* inv_dx2_sum, const double* inv_dx2_levels, double* time, const double* end,
+                     double* dt, int advance, unsigned long long* scratch, cudaStream_t stream);
+
 // dt[i] = min(cfl / rate_i, diffusion limit_i, remaining_i); advances time[i] by it. The
 // diffusion limit is per level when level_keys / inv_dx2_levels are given.
 int launch_finalize_dt(const unsigned long long* keys, int ninstances, double cfl, double diffusivity,

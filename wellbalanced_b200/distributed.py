@@ -535,6 +535,11 @@ class DistributedEngine(Engine):
             self.transport.reduce_min_keys(self.level_keys)
         Engine.finalize_dt(self, cfl, eta, kappa, clip_to_end=clip_to_end, advance=advance)
 
+    def stable_dt(self, cfl, eta=0.0, kappa=0.0, *, advance=False):
+        # the keys are reduced over the ranks between the rate and the dt
+        self.rate()
+        self.finalize_dt(cfl, eta, kappa, advance=advance)
+
     def step(self, cfl):
         """One Heun step of this rank's patches at the global stable dt."""
         self.rate()

@@ -114,6 +114,12 @@ class Engine:
         self.ninstances = n
         self.dt = torch.zeros(n, dtype=torch.float64, device=self.device)
         self.keys = torch.zeros(2 * n, dtype=torch.int64, device=self.device)
+        #: scratch of `stable_dt`: a ticket and the identities of the keys (largest rate 0,
+        #: smallest density +inf per instance and per level), as every launch leaves them
+        identities = np.full(1 + 2 * n + n * self.nlevels, 0xFFF0000000000000, dtype=np.uint64)
+        identities[0] = 0
+        identities[1 : 1 + 2 * n : 2] = 0x8000000000000000
+        self.dt_scratch = torch.from_numpy(identities.view(np.int64)).to(self.device)
         self.time = torch.zeros(n, dtype=torch.float64, device=self.device)
         self.end = torch.zeros(n, dtype=torch.float64, device=self.device)
         self.bad = torch.zeros(1, dtype=torch.int64, device=self.device)
@@ -295,6 +301,18 @@ class Engine:
             _lib.call("wb_finalize_dt", self.keys.data_ptr(), self.ninstances, float(cfl), float(eta), float(kappa),
                       self.gamma, self.inv_dx2_sum.data_ptr(), self.time.data_ptr(), end, self.dt.data_ptr(),
                       int(advance), self._s())
+        self.launches += 1
+
+    def stable_dt(self, cfl, eta=0.0, kappa=0.0, *, advance=False):
+        """`rate` of the state and `finalize_dt` in one launch."""
+        b = self.mean_field
+        levels = self.per_level_dt
+        _lib.call("wb_stable_dt", self.precision, self.ndim, self.state.data_ptr(), self.patches.data_ptr(),
+                  self.chunk_patch.data_ptr(), self.chunk_start.data_ptr(), self.nchunks, b[0], b[1], b[2], self.gamma,
+                  self.keys.data_ptr(), self.ninstances, self.level_keys.data_ptr() if levels else None,
+                  self.nlevels if levels else 0, float(cfl), float(eta), float(kappa), self.inv_dx2_sum.data_ptr(),
+                  self.inv_dx2_levels.data_ptr() if levels else None, self.time.data_ptr(), None, self.dt.data_ptr(),
+                  int(advance), self.dt_scratch.data_ptr(), self._s())
         self.launches += 1
 
     def rate_values(self):
@@ -505,8 +523,7 @@ class Engine:
     def prime_dt(self, cfl, eta=0.0, kappa=0.0):
         """dt of the next programmed step from the current state (time not advanced)."""
         with self.launching():
-            self.rate()
-            self.finalize_dt(cfl, eta, kappa, advance=False)
+            self.stable_dt(cfl, eta, kappa)
         self.dt_ready = True
 
     def programmed_step(self, groups_potential, groups_all, cfl, eta=0.0, kappa=0.0):

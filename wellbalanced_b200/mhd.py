@@ -352,8 +352,7 @@ class MHD2D:
         """The largest stable step (``carafe/mhd.py:930-963``)."""
         self._check_ready()
         eng = self.engine
-        eng.rate()
-        eng.finalize_dt(self.cfl, self.resistivity, max(self.conduction))
+        eng.stable_dt(self.cfl, self.resistivity, max(self.conduction))
         return float(eng.dt[0].item())
 
     def _raise_if_bad(self):
@@ -400,8 +399,7 @@ class MHD2D:
             eng.programmed_step(self._groups_potential, self._groups_all, self.cfl, self.resistivity, max(self.conduction))
             return
         with eng.launching():
-            eng.rate()
-            eng.finalize_dt(self.cfl, self.resistivity, max(self.conduction), advance=True)
+            eng.stable_dt(self.cfl, self.resistivity, max(self.conduction), advance=True)
             eng.heun_step(self._groups_potential, self._groups_all)
 
     def _prime(self):

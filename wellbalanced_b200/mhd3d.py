@@ -309,8 +309,7 @@ class MHD3D:
     def stable_step(self) -> float:
         self._check_ready()
         eng = self.engine
-        eng.rate()
-        eng.finalize_dt(self.cfl, self.resistivity, 0.0)
+        eng.stable_dt(self.cfl, self.resistivity, 0.0)
         return float(eng.dt[0].item())
 
     def _raise_if_bad(self):
@@ -355,8 +354,7 @@ class MHD3D:
             eng.programmed_step(self._groups_potential, self._groups_all, self.cfl, self.resistivity, 0.0)
             return
         with eng.launching():
-            eng.rate()
-            eng.finalize_dt(self.cfl, self.resistivity, 0.0, advance=True)
+            eng.stable_dt(self.cfl, self.resistivity, 0.0, advance=True)
             eng.heun_step(self._groups_potential, self._groups_all)
 
     def _prime(self):

@@ -405,8 +405,7 @@ class PlainMHD3D(MHD3D):
     def stable_step(self):
         self._check_ready()
         eng = self.engine
-        eng.rate()
-        eng.finalize_dt(self.cfl, self.resistivity, 0.0)
+        eng.stable_dt(self.cfl, self.resistivity, 0.0)
         return float(eng.dt[0].item())
 
     def step(self, dt=None):
