@@ -358,6 +358,20 @@ int wb_mlp_backward(const float* features, const float* targets, int64_t n, cons
 int wb_mlp_adam(float* params, float* grads, float* m, float* v, int count, float lr, float beta1, float beta2,
                 float eps, int step, float scale, void* stream);
 
+/* A list of the calls above, issued in order by one call. `code`: wb_launch_code of the
+ * function's name (also "record_event" (event), "wait_event" (event) and "clear_bytes"
+ * (pointer, bytes)); `args`: its arguments before the stream, one per slot, doubles by their
+ * bits; own_stream != 0: launched on `stream`, else on the stream wb_run_launches is given.
+ * The pointers must stay valid while the list is used. The list is run `repeat` times. */
+typedef struct {
+  int32_t code;
+  int32_t own_stream;
+  int64_t stream;
+  int64_t args[26];
+} wb_launch;
+int wb_launch_code(const char* name);
+int wb_run_launches(const void* launches, int count, int repeat, void* stream);
+
 /* wb_rate without a caller-provided key buffer: allocates nothing. No counterpart in the
  * reference (its rate kernel returns into a caller-allocated out[2]). Same work list and
  * state as wb_rate; the per-instance keys live in a static device array of 4096

@@ -49,6 +49,8 @@ SIGNATURES = {
     "wb_finalize_dt": [c_dp, c_int, c_double, c_double, c_double, c_double, c_dp, c_dp, c_dp, c_dp, c_int, c_dp],
     "wb_stable_dt": [c_int, c_int, c_dp, c_dp, c_dp, c_dp, c_int, c_double, c_double, c_double, c_double, c_dp, c_int,
                      c_dp, c_int, c_double, c_double, c_double, c_dp, c_dp, c_dp, c_dp, c_dp, c_int, c_dp, c_dp],
+    "wb_launch_code": [ctypes.c_char_p],
+    "wb_run_launches": [c_dp, c_int, c_int, c_dp],
     "wb_rate_levels": [c_int, c_int, c_dp, c_dp, c_int, c_dp, c_dp, c_int, c_double, c_double, c_double, c_double,
                        c_dp, c_int, c_dp, c_int, c_dp],
     "wb_finalize_dt_levels": [c_dp, c_int, c_double, c_double, c_double, c_double, c_dp, c_dp, c_int, c_dp, c_dp,
@@ -153,6 +155,36 @@ def call(name, *args):
     if status != 0:
         raise WBError(f"{name}: status {status}: {load().wb_last_error().decode()}")
     return status
+
+
+#: one entry of a launch list (wb_launch): code, own_stream, stream, argument slots
+LAUNCH = np.dtype([("code", "<i4"), ("own_stream", "<i4"), ("stream", "<i8"), ("args", "<i8", (26,))])
+#: argument types of the launch-list entries that are no C-ABI functions of their own
+_LAUNCH_ARGS = {"record_event": [c_dp, c_dp], "wait_event": [c_dp, c_dp], "clear_bytes": [c_dp, c_i64, c_dp]}
+_LAUNCH_CODES: dict[str, int] = {}
+
+
+def launch_list(calls):
+    """The C-ABI calls ``(name, args before the stream, stream or None for the one of the run)``
+    as a `LAUNCH` array for ``wb_run_launches``."""
+    out = np.zeros(len(calls), dtype=LAUNCH)
+    for row, (name, args, stream) in zip(out, calls, strict=True):
+        code = _LAUNCH_CODES.get(name)
+        if code is None:
+            code = load().wb_launch_code(name.encode())
+            if code < 0:
+                raise WBError(load().wb_last_error().decode())
+            _LAUNCH_CODES[name] = code
+        types = (SIGNATURES.get(name) or _LAUNCH_ARGS[name])[:-1]
+        if len(types) != len(args):
+            raise ValueError(f"{name}: {len(args)} arguments, {len(types)} expected")
+        row["code"] = code
+        row["own_stream"] = stream is not None
+        row["stream"] = stream or 0
+        slots = [int(np.float64(a).view(np.int64)) if t is c_double else int(a or 0)
+                 for a, t in zip(args, types, strict=True)]
+        row["args"][: len(slots)] = slots
+    return out
 
 
 def tile_shapes_2d(precision) -> list[tuple[int, int]]:

@@ -124,12 +124,9 @@ class Batch:
         return int(sum(nx * ny for nx, ny in self.sides))
 
     # stepping ------------------------------------------------------------------------------------
-    def _step_launches(self):
-        eng = self.engine
-        groups = eng.layout.groups
-        with eng.launching():
-            eng.stable_dt(self.cfl, advance=True)
-            eng.heun_step(groups[1:], groups)
+    def _step_launches(self, steps=1):
+        groups = self.engine.layout.groups
+        self.engine.run_steps(steps, groups[1:], groups, (self.cfl, 0.0, 0.0))
 
     def capture(self):
         """Capture one step (all launches) in a CUDA graph; `advance` then replays it. The
@@ -142,11 +139,11 @@ class Batch:
         eng = self.engine
         if check:
             eng.bad.zero_()
-        for _ in range(steps):
-            if self._graph is not None:
+        if self._graph is not None:
+            for _ in range(steps):
                 self._graph.replay()
-            else:
-                self._step_launches()
+        else:
+            self._step_launches(steps)
         self.steps += steps
         if check and int(eng.bad.item()):
             raise FloatingPointError("non-positive density or pressure (or non-finite values) in the batch")

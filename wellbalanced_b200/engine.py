@@ -112,7 +112,10 @@ class Engine:
                 self.restrict_merged[level] = (frozenset(groups), *upload(ops, _lib.RESTRICT_OP))
         n = L.ninstances
         self.ninstances = n
-        self.dt = torch.zeros(n, dtype=torch.float64, device=self.device)
+        #: what the host reads after a step, in one copy (`read_status`): the bad-cell count,
+        #: then every instance's time and dt by their bits
+        self.status = torch.zeros(1 + 2 * n, dtype=torch.int64, device=self.device)
+        self.dt = self.status[1 + n :].view(torch.float64)
         self.keys = torch.zeros(2 * n, dtype=torch.int64, device=self.device)
         #: scratch of `stable_dt`: a ticket and the identities of the keys (largest rate 0,
         #: smallest density +inf per instance and per level), as every launch leaves them
@@ -120,9 +123,9 @@ class Engine:
         identities[0] = 0
         identities[1 : 1 + 2 * n : 2] = 0x8000000000000000
         self.dt_scratch = torch.from_numpy(identities.view(np.int64)).to(self.device)
-        self.time = torch.zeros(n, dtype=torch.float64, device=self.device)
+        self.time = self.status[1 : 1 + n].view(torch.float64)
         self.end = torch.zeros(n, dtype=torch.float64, device=self.device)
-        self.bad = torch.zeros(1, dtype=torch.int64, device=self.device)
+        self.bad = self.status[:1]
         #: the 2D stage kernel's boundary-face fluxes (float64, allocated on first use): the
         #: register reads the fine faces there instead of recomputing them
         self.bflux = None
@@ -154,6 +157,10 @@ class Engine:
         self._flux_events = None
         #: the launching stream's handle while a step issues its launches (looked up once)
         self._step_stream = None
+        #: the list that launches are put into instead of being issued, and the launch lists
+        #: kept by step (`run_steps`); any other attribute that is set drops them
+        self._recording = None
+        self._lists = {}
         #: run the reflux, restriction, halo-fill and stable-step phases between the stage
         #: kernels as op programs (`wb_run_program`, one launch each: six launches per
         #: refined step instead of ~26). Off by default: on the B200 the separate launches
@@ -166,10 +173,26 @@ class Engine:
         self.dt_ready = False
 
     # low-level launches ----------------------------------------------------------------------
+    #: attributes that launches read nothing from: setting them keeps the launch lists
+    _COUNTERS = frozenset(("launches", "dt_ready", "_step_stream", "_recording", "_lists"))
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name not in Engine._COUNTERS:  # another setting or buffer: the lists are out of date
+            object.__setattr__(self, "_lists", {})
+
     def _s(self):
         if self._step_stream is not None:
             return self._step_stream
         return self._main().cuda_stream
+
+    def _launch(self, name, *args, stream=None):
+        """One C-ABI call, `args` before the stream, on `stream` or the engine's; while a
+        launch list is put together, an entry of it."""
+        if self._recording is not None:
+            self._recording.append((name, args, None if stream is None else stream.cuda_stream))
+        else:
+            _lib.call(name, *args, self._s() if stream is None else stream.cuda_stream)
 
     def _main(self):
         return self.stream if self.stream is not None else torch.cuda.current_stream(self.device)
@@ -183,25 +206,24 @@ class Engine:
     def _fill_level(self, pool, level):
         """Interpolation from the level below, same-level copies, boundary faces."""
         prec = self.precision
-        s = self._s()
         same, nsame, boundary = self.copy_phases[level]
         interp, ninterp = self.interp_levels[level]
         if ninterp and nsame and self.fused_fill:
             # the layout's interpolation ops skip the points the copies write: one launch
-            _lib.call("wb_fill_ops", prec, pool.data_ptr(), self.patches.data_ptr(), interp.data_ptr(), ninterp,
-                      same.data_ptr(), nsame, s)
+            self._launch("wb_fill_ops", prec, pool.data_ptr(), self.patches.data_ptr(), interp.data_ptr(), ninterp,
+                         same.data_ptr(), nsame)
             self.launches += 1
         else:
             if ninterp:
-                _lib.call("wb_interp_ops", prec, pool.data_ptr(), self.patches.data_ptr(), interp.data_ptr(), ninterp,
-                          s)
+                self._launch("wb_interp_ops", prec, pool.data_ptr(), self.patches.data_ptr(), interp.data_ptr(),
+                             ninterp)
                 self.launches += 1
             if nsame:
-                _lib.call("wb_copy_ops", prec, pool.data_ptr(), self.patches.data_ptr(), same.data_ptr(), nsame, s)
+                self._launch("wb_copy_ops", prec, pool.data_ptr(), self.patches.data_ptr(), same.data_ptr(), nsame)
                 self.launches += 1
         for ops, nops in boundary:
             if nops:
-                _lib.call("wb_copy_ops", prec, pool.data_ptr(), self.patches.data_ptr(), ops.data_ptr(), nops, s)
+                self._launch("wb_copy_ops", prec, pool.data_ptr(), self.patches.data_ptr(), ops.data_ptr(), nops)
                 self.launches += 1
 
     def restrict(self, pool, groups):
@@ -212,8 +234,8 @@ class Engine:
             if merged is not None and merged[0] == key:
                 ops, nops = merged[1], merged[2]
                 if nops:
-                    _lib.call("wb_restrict_ops", self.precision, pool.data_ptr(), self.patches.data_ptr(),
-                              ops.data_ptr(), nops, self._s())
+                    self._launch("wb_restrict_ops", self.precision, pool.data_ptr(), self.patches.data_ptr(),
+                                 ops.data_ptr(), nops)
                     self.launches += 1
                 continue
             for g in groups:
@@ -222,8 +244,8 @@ class Engine:
     def _restrict_level(self, pool, level, g):
         ops, nops = self.restrict_levels[level][g]
         if nops:
-            _lib.call("wb_restrict_ops", self.precision, pool.data_ptr(), self.patches.data_ptr(), ops.data_ptr(),
-                      nops, self._s())
+            self._launch("wb_restrict_ops", self.precision, pool.data_ptr(), self.patches.data_ptr(), ops.data_ptr(),
+                         nops)
             self.launches += 1
 
     def _uses_staged_fluxes(self):
@@ -238,7 +260,6 @@ class Engine:
 
     def stage(self, src, base, dst, bflux=None):
         b = self.mean_field
-        s = self._s()
         if self.ntiles == 0:
             return
         if bflux is None and self._uses_staged_fluxes():
@@ -251,28 +272,31 @@ class Engine:
         if self.ndim == 2 and self.physics is not None:
             if tuple(self.layout.tile_shape) != tuple(self.layout.default_tile):
                 raise ValueError("the non-ideal 2D stage kernel runs on the default tile shape")
-            _lib.call("wb_stage2d_physics", self.precision, src.data_ptr(), None if base is None else base.data_ptr(),
-                      dst.data_ptr(), self.patches.data_ptr(), self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(),
-                      self.gamma, b[0], b[1], self.limiter, *self.physics, self.bad.data_ptr(), s)
+            self._launch("wb_stage2d_physics", self.precision, src.data_ptr(),
+                         None if base is None else base.data_ptr(), dst.data_ptr(), self.patches.data_ptr(),
+                         self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(),
+                         self.gamma, b[0], b[1], self.limiter, *self.physics, self.bad.data_ptr())
         elif self.ndim == 2:
             tx, ty = self.layout.tile_shape
-            _lib.call("wb_stage2d_tiled", self.precision, src.data_ptr(), None if base is None else base.data_ptr(),
-                      dst.data_ptr(), self.patches.data_ptr(), self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(),
-                      self.gamma, b[0], b[1], self.limiter, tx, ty, self.bad.data_ptr(),
-                      None if bflux is None else bflux.data_ptr(), s)
+            self._launch("wb_stage2d_tiled", self.precision, src.data_ptr(),
+                         None if base is None else base.data_ptr(), dst.data_ptr(), self.patches.data_ptr(),
+                         self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(),
+                         self.gamma, b[0], b[1], self.limiter, tx, ty, self.bad.data_ptr(),
+                         None if bflux is None else bflux.data_ptr())
         elif self.physics is not None:
             if tuple(self.layout.tile_shape) != tuple(self.layout.default_tile):
                 raise ValueError("the non-ideal 3D stage kernel runs on the default tile shape")
-            _lib.call("wb_stage3d_physics", self.precision, src.data_ptr(),
-                      None if base is None else base.data_ptr(), dst.data_ptr(), self.patches.data_ptr(),
-                      self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(), self.gamma, b[0], b[1], b[2],
-                      self.limiter, self.layout.march, *self.physics, self.bad.data_ptr(), s)
+            self._launch("wb_stage3d_physics", self.precision, src.data_ptr(),
+                         None if base is None else base.data_ptr(), dst.data_ptr(), self.patches.data_ptr(),
+                         self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(), self.gamma, b[0], b[1], b[2],
+                         self.limiter, self.layout.march, *self.physics, self.bad.data_ptr())
         else:
             ty, tz = self.layout.tile_shape
-            _lib.call("wb_stage3d_tiled", self.precision, src.data_ptr(), None if base is None else base.data_ptr(),
-                      dst.data_ptr(), self.patches.data_ptr(), self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(),
-                      self.gamma, b[0], b[1], b[2], self.limiter, self.layout.march, ty, tz, self.bad.data_ptr(),
-                      None if bflux is None else bflux.data_ptr(), s)
+            self._launch("wb_stage3d_tiled", self.precision, src.data_ptr(),
+                         None if base is None else base.data_ptr(), dst.data_ptr(), self.patches.data_ptr(),
+                         self.tiles.data_ptr(), self.ntiles, self.dt.data_ptr(),
+                         self.gamma, b[0], b[1], b[2], self.limiter, self.layout.march, ty, tz, self.bad.data_ptr(),
+                         None if bflux is None else bflux.data_ptr())
         if timing:
             end.record(torch.cuda.current_stream(self.device) if self.stream is None else self.stream)
             self.stage_events.append((start, end))
@@ -307,13 +331,19 @@ class Engine:
         """`rate` of the state and `finalize_dt` in one launch."""
         b = self.mean_field
         levels = self.per_level_dt
-        _lib.call("wb_stable_dt", self.precision, self.ndim, self.state.data_ptr(), self.patches.data_ptr(),
-                  self.chunk_patch.data_ptr(), self.chunk_start.data_ptr(), self.nchunks, b[0], b[1], b[2], self.gamma,
-                  self.keys.data_ptr(), self.ninstances, self.level_keys.data_ptr() if levels else None,
-                  self.nlevels if levels else 0, float(cfl), float(eta), float(kappa), self.inv_dx2_sum.data_ptr(),
-                  self.inv_dx2_levels.data_ptr() if levels else None, self.time.data_ptr(), None, self.dt.data_ptr(),
-                  int(advance), self.dt_scratch.data_ptr(), self._s())
+        self._launch("wb_stable_dt", self.precision, self.ndim, self.state.data_ptr(), self.patches.data_ptr(),
+                     self.chunk_patch.data_ptr(), self.chunk_start.data_ptr(), self.nchunks, b[0], b[1], b[2],
+                     self.gamma, self.keys.data_ptr(), self.ninstances, self.level_keys.data_ptr() if levels else None,
+                     self.nlevels if levels else 0, float(cfl), float(eta), float(kappa), self.inv_dx2_sum.data_ptr(),
+                     self.inv_dx2_levels.data_ptr() if levels else None, self.time.data_ptr(), None, self.dt.data_ptr(),
+                     int(advance), self.dt_scratch.data_ptr())
         self.launches += 1
+
+    def read_status(self):
+        """(bad cells, times, dts) on the host, once the launches so far are done: one copy."""
+        host = self.status.cpu().numpy()
+        n = self.ninstances
+        return int(host[0]), host[1 : 1 + n].view(np.float64), host[1 + n :].view(np.float64)
 
     def rate_values(self):
         """(max rate, min density) per instance, on the host."""
@@ -330,32 +360,31 @@ class Engine:
         (on `stream`, else the engine's stream). `pool` is the input of the stage just
         launched: with staged fluxes its fine faces are read from that stage's output."""
         if self.nface:
-            s = stream.cuda_stream if stream is not None else self._s()
             b = self.mean_field
             if self.physics is not None:
                 eta, kappa_par, kappa_perp = self.physics[:3] if self.ndim == 2 else (self.physics[0], 0.0, 0.0)
             if self.physics is not None and (eta or kappa_par or kappa_perp):
-                _lib.call("wb_face_flux_ops_physics", self.precision, pool.data_ptr(), self.patches.data_ptr(),
-                          self.face_flux_ops.data_ptr(), self.nface, b[0], b[1], b[2], self.gamma, self.limiter, eta,
-                          kappa_par, kappa_perp, self.register.data_ptr(), s)
+                self._launch("wb_face_flux_ops_physics", self.precision, pool.data_ptr(), self.patches.data_ptr(),
+                             self.face_flux_ops.data_ptr(), self.nface, b[0], b[1], b[2], self.gamma, self.limiter, eta,
+                             kappa_par, kappa_perp, self.register.data_ptr(), stream=stream)
             elif self._uses_staged_fluxes():
                 # the fine faces as the stage kernel that read `pool` wrote them
-                _lib.call("wb_face_flux_ops_staged", self.precision, pool.data_ptr(), self.patches.data_ptr(),
-                          self.face_flux_ops.data_ptr(), self.nface, self.nface_faces, b[0], b[1], b[2], self.gamma,
-                          self.limiter, self._stage_bflux().data_ptr(), self.register.data_ptr(), s)
+                self._launch("wb_face_flux_ops_staged", self.precision, pool.data_ptr(), self.patches.data_ptr(),
+                             self.face_flux_ops.data_ptr(), self.nface, self.nface_faces, b[0], b[1], b[2], self.gamma,
+                             self.limiter, self._stage_bflux().data_ptr(), self.register.data_ptr(), stream=stream)
             else:
-                _lib.call("wb_face_flux_ops", self.precision, pool.data_ptr(), self.patches.data_ptr(),
-                          self.face_flux_ops.data_ptr(), self.nface, b[0], b[1], b[2], self.gamma, self.limiter,
-                          self.register.data_ptr(), s)
+                self._launch("wb_face_flux_ops", self.precision, pool.data_ptr(), self.patches.data_ptr(),
+                             self.face_flux_ops.data_ptr(), self.nface, b[0], b[1], b[2], self.gamma, self.limiter,
+                             self.register.data_ptr(), stream=stream)
             self.launches += 1
 
     def reflux(self, pool):
         """Coarse cells beside fine patches take the register's correction (then cleared)."""
         size = _lib.REFLUX_OP.itemsize
         for start, count in self.reflux_phases:
-            _lib.call("wb_reflux_apply", self.precision, pool.data_ptr(), self.patches.data_ptr(),
-                      self.reflux_ops.data_ptr() + start * size, count, self.register.data_ptr(),
-                      self.dt.data_ptr(), self._s())
+            self._launch("wb_reflux_apply", self.precision, pool.data_ptr(), self.patches.data_ptr(),
+                         self.reflux_ops.data_ptr() + start * size, count, self.register.data_ptr(),
+                         self.dt.data_ptr())
             self.launches += 1
 
     def capture(self, step):
@@ -375,9 +404,48 @@ class Engine:
 
     def heun_step(self, groups_potential, groups_all):
         """One Heun step with the dt already in self.dt (device), refluxed and restricted."""
+        self.run_steps(1, groups_potential, groups_all)
+
+    def run_steps(self, count, groups_potential, groups_all, dt_params=None, *, advance=True, clear_bad=False):
+        """`count` Heun steps, each at the dt on the device or, with dt_params (cfl, eta, kappa),
+        at the stable dt of its state (`stable_dt`; the time advanced by it unless not `advance`);
+        with clear_bad the bad-cell count is zeroed before each. The launches of a step are put
+        together once (`_lib.launch_list`) and issued by one native call for all steps; a rank
+        of a partition, whose exchanges run between them, and timed stages issue them one by one."""
         self.dt_ready = False
-        with self.launching():
+
+        def launches():
+            if dt_params is not None:
+                self.stable_dt(*dt_params, advance=advance)
             self._heun_launches(groups_potential, groups_all)
+
+        if type(self) is not Engine or self.stage_events is not None:
+            with self.launching():
+                for _ in range(count):
+                    if clear_bad:
+                        self.bad.zero_()
+                    launches()
+            return
+        key = (tuple(groups_potential), tuple(groups_all), dt_params, advance, clear_bad)
+        found = self._lists.get(key)
+        if found is None:
+            if self.max_level > 0 and self._uses_staged_fluxes():
+                self._stage_bflux()  # allocated before the recording, not by it
+            self._side_stream()
+            before = self.launches
+            self._recording = []
+            try:
+                if clear_bad:
+                    self._launch("clear_bytes", self.bad.data_ptr(), 8)
+                launches()
+                found = (_lib.launch_list(self._recording), self.launches - before)
+            finally:
+                self._recording = None
+                self.launches = before
+            self._lists[key] = found
+        entries, kernels = found
+        _lib.call("wb_run_launches", entries.ctypes.data, int(entries.size), int(count), self._s())
+        self.launches += kernels * count
 
     @contextlib.contextmanager
     def launching(self):
@@ -391,28 +459,43 @@ class Engine:
         finally:
             self._step_stream = outer
 
+    def _side_stream(self):
+        """The flux register's own stream and its fork and join events (made on first use), or
+        None where the register runs with the rest."""
+        if not (self.overlap_fluxes and self.nface):
+            return None
+        if self._flux_stream is None:
+            self._flux_stream = torch.cuda.Stream(self.device)
+            self._flux_events = (torch.cuda.Event(), torch.cuda.Event())
+            for event in self._flux_events:  # an event has its handle from its first record on
+                event.record(self._flux_stream)
+        return self._flux_stream
+
+    def _order(self, event, first, then):
+        """`then` waits for what `first` has issued so far (None: the engine's stream)."""
+        if self._recording is not None:
+            self._launch("record_event", event.cuda_event, stream=first)
+            self._launch("wait_event", event.cuda_event, stream=then)
+            return
+        event.record(self._main() if first is None else first)
+        (self._main() if then is None else then).wait_event(event)
+
     def _heun_launches(self, groups_potential, groups_all):
         U, U1 = self.state, self.stage_pool
         refined = self.max_level > 0
         self.stage(U, None, U1)
-        side = None
-        if self.overlap_fluxes and self.nface:
-            # stage 1's register kernel beside the restriction and fill of U1 (small,
-            # latency-bound launches that leave the SMs idle), not beside the stage kernel
-            if self._flux_stream is None:
-                self._flux_stream = torch.cuda.Stream(self.device)
-                self._flux_events = (torch.cuda.Event(), torch.cuda.Event())
-            side, main = self._flux_stream, self._main()
+        # stage 1's register kernel beside the restriction and fill of U1 (small,
+        # latency-bound launches that leave the SMs idle), not beside the stage kernel
+        side = self._side_stream()
+        if side is not None:
             forked, joined = self._flux_events
-            forked.record(main)
-            side.wait_event(forked)
+            self._order(forked, None, side)
         self.face_fluxes(U, side)
         if refined:
             self.restrict(U1, groups_potential)
         self.fill(U1)
         if side is not None:
-            joined.record(side)
-            main.wait_event(joined)  # stage 1's fluxes have read U before stage 2 writes it
+            self._order(joined, side, None)  # stage 1's fluxes have read U before stage 2 writes it
         self.stage(U1, U, U)
         self.face_fluxes(U1)
         self.reflux(U)
@@ -535,13 +618,10 @@ class Engine:
         with self.launching():
             U, U1 = self.state, self.stage_pool
             self.stage(U, None, U1)
-            side = None
-            if self.overlap_fluxes and self.nface:
-                if self._flux_stream is None:
-                    self._flux_stream = torch.cuda.Stream(self.device)
-                    self._flux_events = (torch.cuda.Event(), torch.cuda.Event())
-                side, main = self._flux_stream, self._main()
+            side = self._side_stream()
+            if side is not None:
                 forked, joined = self._flux_events
+                main = self._main()
                 forked.record(main)
                 side.wait_event(forked)
             self.face_fluxes(U, side)

@@ -355,27 +355,32 @@ class MHD2D:
         eng.stable_dt(self.cfl, self.resistivity, max(self.conduction))
         return float(eng.dt[0].item())
 
-    def _raise_if_bad(self):
+    def _raise_if_bad(self, bad=None):
         if self.engine.use_programs and self.engine.program_error():
             raise RuntimeError("an op program's phase wait ran out (its device error word is set)")
-        if int(self.engine.bad.item()):
+        if int(self.engine.bad.item()) if bad is None else bad:
             raise FloatingPointError(f"non-positive density or pressure (or non-finite values) at t = {self.time}")
 
     def step(self, dt: float | None = None) -> float:
         """Advance by one step of Heun's method (SSP-RK2); return the step taken."""
         self._check_ready()
         eng = self.engine
-        if dt is None:
-            dt = self.stable_step()
-        else:
+        if dt is not None:
             eng.dt.fill_(float(dt))
-        eng.bad.zero_()
-        eng.heun_step(self._groups_potential, self._groups_all)
-        self._raise_if_bad()
-        self.time += float(dt)
+        eng.run_steps(1, self._groups_potential, self._groups_all, self._dt_params() if dt is None else None,
+                      advance=False, clear_bad=True)
+        # the one wait of the step: its dt and its bad cells together
+        bad, _, taken = eng.read_status()
+        self._raise_if_bad(bad)
+        dt = float(taken[0]) if dt is None else float(dt)
+        self.time += dt
         self.steps += 1
         eng.time.fill_(self.time)
-        return float(dt)
+        return dt
+
+    def _dt_params(self):
+        """(cfl, resistivity, conductivity) of the stable step."""
+        return self.cfl, self.resistivity, max(self.conduction)
 
     def run(self, duration: float, *, max_steps: int = 1_000_000) -> int:
         """Advance by ``duration`` (the last step shortened to land on it); return the steps."""
@@ -398,9 +403,7 @@ class MHD2D:
         if eng.use_programs:
             eng.programmed_step(self._groups_potential, self._groups_all, self.cfl, self.resistivity, max(self.conduction))
             return
-        with eng.launching():
-            eng.stable_dt(self.cfl, self.resistivity, max(self.conduction), advance=True)
-            eng.heun_step(self._groups_potential, self._groups_all)
+        eng.run_steps(1, self._groups_potential, self._groups_all, self._dt_params())
 
     def _prime(self):
         if self.engine.use_programs and not self.engine.dt_ready:
@@ -423,15 +426,19 @@ class MHD2D:
         eng = self.engine
         eng.bad.zero_()
         self._prime()
-        for _ in range(steps):
-            if self._graph is not None:
-                self._graph.replay()
-            else:
-                self._one_step()
+        if self._graph is None and not eng.use_programs:
+            eng.run_steps(steps, self._groups_potential, self._groups_all, self._dt_params())
+        else:
+            for _ in range(steps):
+                if self._graph is not None:
+                    self._graph.replay()
+                else:
+                    self._one_step()
         self.steps += steps
         if check:
-            self.time = float(eng.time[0].item())
-            self._raise_if_bad()
+            bad, time, _ = eng.read_status()
+            self.time = float(time[0])
+            self._raise_if_bad(bad)
 
     def save(self, host=None):
         """Copy the device state pool into ``host`` (a pinned CPU tensor, allocated if None);
