@@ -56,60 +56,114 @@ __device__ __forceinline__ void cell_quantities(const S* src, const PatchDesc& P
   q[2] = sqrtf(float(bx * bx + by * by + bz * bz));
 }
 
-// One thread per interior cell (work list of the rate kernels: up to 2048 cells per chunk).
 // Features of a cell from its 3 x 3 x 3 neighbourhood, for each of (log rho, log p, |B|):
 // the value, the three central differences (half the difference of the two neighbours
 // along an axis) and the largest deviation over the 26 neighbours; feature 15 is zero.
 // Output row t of a patch's block is its cell (i, j, k) in (i, j, k) order, normalised
-// as (f - mean) * inv_std.
+// as (f - mean) * inv_std. Work list of the rate kernels: up to 2048 cells per chunk.
+//
+// The quantities of a cell (two logarithms, a root, the float64 pressure, 17 loads) are what a
+// cell costs: forming those of all 27 neighbours by every thread took 27 of them a row. A
+// block takes 512 consecutive cells, forms each quantity of their neighbourhood once in
+// shared memory (about 4 a row) and then the stencils. The neighbourhood is the box of
+// planes, rows and whole z-lines around the cells where that fits the 72 KB (three blocks of
+// 512 threads an SM): z up to 510 cells inside one plane, patches of up to 24 x 24 across
+// planes; other cells go row by row, three lines of three rows each.
+// B200, 491,000 cells in 203 patches: 195 -> 50 us.
+constexpr int kTagCells = 512;
+constexpr int kTagRegion = 6144;  // cells of the neighbourhood held at once
+constexpr size_t kTagSmem = 3 * kTagRegion * sizeof(float);
+
 template <typename S>
-__global__ void __launch_bounds__(256) tag_features3d_kernel(const S* __restrict__ pool, const PatchDesc* patches,
-                                                             const int* chunk_patch, const int* chunk_start,
-                                                             const int64_t* row_start, double b0x, double b0y,
-                                                             double b0z, double gamma, const float* mean,
-                                                             const float* inv_std, float* __restrict__ out) {
-  const int pi = chunk_patch[blockIdx.x];
+__global__ void __launch_bounds__(kTagCells) tag_features3d_kernel(const S* __restrict__ pool, const PatchDesc* patches,
+                                                                   const int* chunk_patch, const int* chunk_start,
+                                                                   const int64_t* row_start, double b0x, double b0y,
+                                                                   double b0z, double gamma, const float* mean,
+                                                                   const float* inv_std, float* __restrict__ out) {
+  extern __shared__ float q[];  // [3][kTagRegion]
+  constexpr int kParts = 2048 / kTagCells;
+  const int chunk = int(blockIdx.x) / kParts, part = int(blockIdx.x) % kParts;
+  const int pi = chunk_patch[chunk];
   const PatchDesc P = patches[pi];
   const int nx = P.n[0], ny = P.n[1], nz = P.n[2];
   const S* src = pool + P.off;
   const double b0[3] = {b0x, b0y, b0z};
   const unsigned total = unsigned(nx) * unsigned(ny) * unsigned(nz);
-  const unsigned start = unsigned(chunk_start[blockIdx.x]);
-  for (int s = 0; s < 8; ++s) {
-    const unsigned t = start + unsigned(s) * blockDim.x + threadIdx.x;
-    if (t >= total) break;
-    const unsigned line = t / unsigned(nz);
-    const unsigned plane = line / unsigned(ny);
-    const int i = int(plane) + kHalo, j = int(line - plane * unsigned(ny)) + kHalo,
-              k = int(t - line * unsigned(nz)) + kHalo;
-    float q[3][3][3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int b = 0; b < 3; ++b)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) cell_quantities<S>(src, P, i + a - 1, j + b - 1, k + c - 1, b0, gamma, q[a][b][c]);
-    float f[kFeat];
-#pragma unroll
-    for (int v = 0; v < 3; ++v) {
-      const float c0 = q[1][1][1][v];
-      float dev = 0.0f;
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) dev = fmaxf(dev, fabsf(q[a][b][c][v] - c0));
-      f[v] = c0;
-      f[3 + 3 * v + 0] = 0.5f * (q[2][1][1][v] - q[0][1][1][v]);
-      f[3 + 3 * v + 1] = 0.5f * (q[1][2][1][v] - q[1][0][1][v]);
-      f[3 + 3 * v + 2] = 0.5f * (q[1][1][2][v] - q[1][1][0][v]);
-      f[12 + v] = dev;
+  const unsigned begin = unsigned(chunk_start[chunk]) + unsigned(part) * kTagCells;
+  if (begin >= total) return;
+  const unsigned end = min(begin + unsigned(kTagCells), total);
+  for (unsigned first = begin; first < end;) {
+    // the segment [first, last) and its box of neighbours: planes i0 - 1 .. i1 + 1, rows
+    // j0 - 1 .. j1 + 1, cells k0 - 1 .. k1 + 1 of the interior indices
+    unsigned last = end;
+    const unsigned line0 = first / unsigned(nz);
+    unsigned line1 = (last - 1) / unsigned(nz);
+    int i0 = int(line0 / unsigned(ny)), j0 = int(line0 - unsigned(i0) * unsigned(ny)), k0 = 0;
+    int i1 = int(line1 / unsigned(ny)), j1 = int(line1 - unsigned(i1) * unsigned(ny)), k1 = nz - 1;
+    if (i1 > i0) j1 = ny - 1;
+    const int jb = i1 > i0 ? 0 : j0;
+    int64_t cells = int64_t(i1 - i0 + 3) * (j1 - jb + 3) * (int64_t(nz) + 2);
+    if (cells <= kTagRegion) {
+      j0 = jb;
+    } else {  // one row at a time, its part of the line only
+      last = min(end, (line0 + 1) * unsigned(nz));
+      i1 = i0;
+      j1 = j0;
+      k0 = int(first - line0 * unsigned(nz));
+      k1 = int(last - 1 - line0 * unsigned(nz));
+      cells = int64_t(3) * 3 * (k1 - k0 + 3);  // at most 9 x 514
     }
-    f[15] = 0.0f;
-    float* row = out + (row_start[pi] + int64_t(t)) * kFeat;
+    const int width = k1 - k0 + 3, rows = j1 - j0 + 3;
+    for (int t = threadIdx.x; t < int(cells); t += kTagCells) {
+      const int line = t / width, k = t - line * width;
+      const int plane = line / rows, j = line - plane * rows;
+      float v[3];
+      cell_quantities<S>(src, P, i0 - 1 + plane + kHalo, j0 - 1 + j + kHalo, k0 - 1 + k + kHalo, b0, gamma, v);
+      q[t] = v[0];
+      q[kTagRegion + t] = v[1];
+      q[2 * kTagRegion + t] = v[2];
+    }
+    __syncthreads();
+    const unsigned t = first + threadIdx.x;
+    if (t < last) {
+      const unsigned line = t / unsigned(nz);
+      const int i = int(line / unsigned(ny));
+      const int j = int(line - unsigned(i) * unsigned(ny)), k = int(t - line * unsigned(nz));
+      const int at = ((i - i0 + 1) * rows + (j - j0 + 1)) * width + (k - k0 + 1);
+      const int sj = width, si = rows * width;
+      float f[kFeat];
 #pragma unroll
-    for (int c = 0; c < kFeat; ++c) row[c] = (f[c] - mean[c]) * inv_std[c];
+      for (int v = 0; v < 3; ++v) {
+        const float* c = q + v * kTagRegion + at;
+        const float c0 = c[0];
+        float dev = 0.0f;
+#pragma unroll
+        for (int a = -1; a <= 1; ++a)
+#pragma unroll
+          for (int b = -1; b <= 1; ++b)
+#pragma unroll
+            for (int d = -1; d <= 1; ++d) dev = fmaxf(dev, fabsf(c[a * si + b * sj + d] - c0));
+        f[v] = c0;
+        f[3 + 3 * v + 0] = 0.5f * (c[si] - c[-si]);
+        f[3 + 3 * v + 1] = 0.5f * (c[sj] - c[-sj]);
+        f[3 + 3 * v + 2] = 0.5f * (c[1] - c[-1]);
+        f[12 + v] = dev;
+      }
+      f[15] = 0.0f;
+      float* row = out + (row_start[pi] + int64_t(t)) * kFeat;
+#pragma unroll
+      for (int c = 0; c < kFeat; ++c) f[c] = (f[c] - mean[c]) * inv_std[c];
+      if ((reinterpret_cast<uintptr_t>(out) & 15) == 0) {  // uniform: rows are 64 bytes
+#pragma unroll
+        for (int c = 0; c < kFeat; c += 4)
+          *reinterpret_cast<float4*>(row + c) = make_float4(f[c], f[c + 1], f[c + 2], f[c + 3]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < kFeat; ++c) row[c] = f[c];
+      }
+    }
+    __syncthreads();
+    first = last;
   }
 }
 
@@ -398,16 +452,18 @@ extern "C" int wb_tag_features(int precision, const void* pool, const void* patc
   }
   if (nchunks <= 0) return kOk;
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (precision == 32)
-    tag_features3d_kernel<float><<<nchunks, 256, 0, s>>>(static_cast<const float*>(pool),
-                                                         static_cast<const PatchDesc*>(patches), chunk_patch,
-                                                         chunk_start, row_start, b0x, b0y, b0z, gamma, mean,
-                                                         inv_std, out);
-  else if (precision == 64 || precision == kMath32State64)  // a float64 state
-    tag_features3d_kernel<double><<<nchunks, 256, 0, s>>>(static_cast<const double*>(pool),
-                                                          static_cast<const PatchDesc*>(patches), chunk_patch,
-                                                          chunk_start, row_start, b0x, b0y, b0z, gamma, mean,
-                                                          inv_std, out);
+  const int grid = nchunks * (2048 / kTagCells);
+  if (precision == 32) {
+    cudaFuncSetAttribute(tag_features3d_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTagSmem));
+    tag_features3d_kernel<float><<<grid, kTagCells, kTagSmem, s>>>(
+        static_cast<const float*>(pool), static_cast<const PatchDesc*>(patches), chunk_patch, chunk_start, row_start,
+        b0x, b0y, b0z, gamma, mean, inv_std, out);
+  } else if (precision == 64 || precision == kMath32State64) {  // a float64 state
+    cudaFuncSetAttribute(tag_features3d_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTagSmem));
+    tag_features3d_kernel<double><<<grid, kTagCells, kTagSmem, s>>>(
+        static_cast<const double*>(pool), static_cast<const PatchDesc*>(patches), chunk_patch, chunk_start, row_start,
+        b0x, b0y, b0z, gamma, mean, inv_std, out);
+  }
   else {
     set_error("tag_features: precision is 32, 64 or %d, not %d", kMath32State64, precision);
     return kBadArgument;
