@@ -31,6 +31,16 @@ struct StageArgs {
   double gravity[3] = {0.0, 0.0, 0.0};
 };
 
+// The images of interior point g of a periodic axis of n points in the halo: g + n where g
+// lies among the first `first` points (2 cells, or 3 nodes: the halo's upper side), g - n
+// among the last two. f(offset) with each offset from g, 0 first.
+template <typename F>
+__device__ __forceinline__ void for_axis_images(int g, int n, int first, F f) {
+  f(0);
+  if (g < first) f(n);
+  if (g >= n - 2) f(-n);
+}
+
 // The precision code of a float64 state advanced with float32 arithmetic (the C ABI's
 // WB_MATH32_STATE64); the other codes are 32 (float32 state and arithmetic) and 64.
 constexpr int kMath32State64 = 6432;

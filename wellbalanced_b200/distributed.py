@@ -36,7 +36,7 @@ import torch
 
 from wellbalanced_b200 import _lib
 from wellbalanced_b200.engine import Engine, _device_bytes
-from wellbalanced_b200.mesh import _concat, size_ops, split_box_ops
+from wellbalanced_b200.mesh import WRAP, _concat, size_ops, split_box_ops
 
 #: patch-row flag of a dense block that stands for a box of a patch (kProxy in layout.cuh)
 PROXY = 1 << 30
@@ -209,6 +209,7 @@ class RankLayout:
         self.precision = layout.precision
         self.lx = layout.lx
         self.march = layout.march
+        self.wraps = False
         self.tile_shape = layout.tile_shape
         self.default_tile = getattr(layout, "default_tile", layout.tile_shape)
         self.walls = layout.walls
@@ -225,6 +226,7 @@ class RankLayout:
             r["off"] = offset
             r["instance"] = 0
             r["bflux"] = -1
+            r["flags"] &= ~WRAP  # the exchange rounds fill the halos
             offset += int(r["fstride"]) * self.nfields
         # proxies address their blocks through the source's haloed coordinates: keep the
         # mailboxes above the largest shift that needs, so every row offset stays >= 0

@@ -493,7 +493,8 @@ class Engine:
         self.face_fluxes(U, side)
         if refined:
             self.restrict(U1, groups_potential)
-        self.fill(U1)
+        if not self.layout.wraps:  # else the stage has written U1's halo
+            self.fill(U1)
         if side is not None:
             self._order(joined, side, None)  # stage 1's fluxes have read U before stage 2 writes it
         self.stage(U1, U, U)
@@ -501,7 +502,8 @@ class Engine:
         self.reflux(U)
         if refined:
             self.restrict(U, groups_all)
-        self.fill(U)
+        if not self.layout.wraps:
+            self.fill(U)
 
     # op programs ------------------------------------------------------------------------------
     def _fill_phases(self, pool):
