@@ -29,6 +29,7 @@ namespace wb {
 template <typename S>
 __global__ void __launch_bounds__(kOpThreads) copy_ops_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
                                                              const CopyOp* __restrict__ ops) {
+  after_previous();
   copy_op_pairs(pool, patches, ops[blockIdx.x]);
 }
 
@@ -40,6 +41,7 @@ template <typename S>
 __global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>) interp_ops_kernel(S* __restrict__ pool,
                                                                const PatchDesc* __restrict__ patches,
                                                                const InterpOp* __restrict__ ops) {
+  after_previous();
   interp_op(pool, patches, ops[blockIdx.x]);
 }
 
@@ -51,6 +53,7 @@ template <typename S>
 __global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>) fill_ops_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
                                                              const InterpOp* __restrict__ interp, int ninterp,
                                                              const CopyOp* __restrict__ copies) {
+  after_previous();
   if (int(blockIdx.x) < ninterp)
     interp_op(pool, patches, interp[blockIdx.x]);
   else
@@ -61,30 +64,31 @@ template <typename S>
 __global__ void __launch_bounds__(kOpThreads) restrict_ops_kernel(S* __restrict__ pool,
                                                                  const PatchDesc* __restrict__ patches,
                                                                  const RestrictOp* __restrict__ ops) {
+  after_previous();
   restrict_op(pool, patches, ops[blockIdx.x]);
 }
 
 template <typename S>
 int launch_copy_ops(S* pool, const PatchDesc* patches, const CopyOp* ops, int nops, cudaStream_t stream) {
-  if (nops > 0) copy_ops_kernel<S><<<nops, kOpThreads, 0, stream>>>(pool, patches, ops);
+  if (nops > 0) launch_after(copy_ops_kernel<S>, nops, kOpThreads, 0, stream, pool, patches, ops);
   return check_launch("halo copy");
 }
 template <typename S>
 int launch_interp_ops(S* pool, const PatchDesc* patches, const InterpOp* ops, int nops, cudaStream_t stream) {
-  if (nops > 0) interp_ops_kernel<S><<<nops, kOpThreads, 0, stream>>>(pool, patches, ops);
+  if (nops > 0) launch_after(interp_ops_kernel<S>, nops, kOpThreads, 0, stream, pool, patches, ops);
   return check_launch("halo interpolation");
 }
 template <typename S>
 int launch_fill_ops(S* pool, const PatchDesc* patches, const InterpOp* interp, int ninterp, const CopyOp* copies,
                     int ncopies, cudaStream_t stream) {
   if (ninterp + ncopies > 0)
-    fill_ops_kernel<S><<<ninterp + ncopies, kOpThreads, 0, stream>>>(pool, patches, interp, ninterp, copies);
+    launch_after(fill_ops_kernel<S>, ninterp + ncopies, kOpThreads, 0, stream, pool, patches, interp, ninterp, copies);
   return check_launch("halo fill");
 }
 
 template <typename S>
 int launch_restrict_ops(S* pool, const PatchDesc* patches, const RestrictOp* ops, int nops, cudaStream_t stream) {
-  if (nops > 0) restrict_ops_kernel<S><<<nops, kOpThreads, 0, stream>>>(pool, patches, ops);
+  if (nops > 0) launch_after(restrict_ops_kernel<S>, nops, kOpThreads, 0, stream, pool, patches, ops);
   return check_launch("restrict");
 }
 template int launch_copy_ops<float>(float*, const PatchDesc*, const CopyOp*, int, cudaStream_t);

@@ -281,6 +281,7 @@ __global__ void __launch_bounds__(kFluxThreads) face_flux_ops_kernel(const S* __
                                                                      const FaceFluxOp* __restrict__ ops, int nops,
                                                                      int splits, double b0x, double b0y, double b0z, double gamma,
                                                                      FacePhysics phys, double* __restrict__ reg) {
+  after_previous();
   __shared__ double g_all[kFluxWarps][32][6];
   const int warp = threadIdx.x / 32, t = threadIdx.x % 32;
   const int item = blockIdx.x * kFluxWarps + warp, index = item / splits;
@@ -329,6 +330,7 @@ template <typename S>
 __global__ void reflux_apply_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
                                     const RefluxOp* __restrict__ ops, double* __restrict__ reg,
                                     const double* __restrict__ dt) {
+  after_previous();
   reflux_op<S, 128>(pool, patches, ops[blockIdx.x], reg, dt);
 }
 
@@ -345,6 +347,7 @@ __global__ void __launch_bounds__(kStagedThreads) face_flux_staged_kernel(
     const S* __restrict__ pool, const PatchDesc* __restrict__ patches, const FaceFluxOp* __restrict__ ops, int nops,
     int nfaces, double b0x, double b0y, double b0z, double gamma, const double* __restrict__ bflux,
     double* __restrict__ reg) {
+  after_previous();
   const int face = blockIdx.x * kStagedThreads + threadIdx.x;
   if (face >= nfaces) return;
   // the op holding this face: the last one whose first face is not after it
@@ -386,10 +389,10 @@ void launch_face_flux_staged(const S* pool, const PatchDesc* patches, const Face
   if (nfaces <= 0) return;
   const int grid = (nfaces + kStagedThreads - 1) / kStagedThreads;
   switch (limiter) {
-    case 0: face_flux_staged_kernel<S, R, 0><<<grid, kStagedThreads, 0, stream>>>(pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
-    case 1: face_flux_staged_kernel<S, R, 1><<<grid, kStagedThreads, 0, stream>>>(pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
-    case 2: face_flux_staged_kernel<S, R, 2><<<grid, kStagedThreads, 0, stream>>>(pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
-    default: face_flux_staged_kernel<S, R, 3><<<grid, kStagedThreads, 0, stream>>>(pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
+    case 0: launch_after(face_flux_staged_kernel<S, R, 0>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
+    case 1: launch_after(face_flux_staged_kernel<S, R, 1>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
+    case 2: launch_after(face_flux_staged_kernel<S, R, 2>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
+    default: launch_after(face_flux_staged_kernel<S, R, 3>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
   }
 }
 
@@ -400,10 +403,10 @@ void launch_face_flux_kernel(const S* pool, const PatchDesc* patches, const Face
   const int splits = flux_splits(nops);
   const int grid = int((int64_t(nops) * splits + kFluxWarps - 1) / kFluxWarps);
   switch (limiter) {
-    case 0: face_flux_ops_kernel<S, R, 0, PHYS><<<grid, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    case 1: face_flux_ops_kernel<S, R, 1, PHYS><<<grid, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    case 2: face_flux_ops_kernel<S, R, 2, PHYS><<<grid, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    default: face_flux_ops_kernel<S, R, 3, PHYS><<<grid, kFluxThreads, 0, stream>>>(pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    case 0: launch_after(face_flux_ops_kernel<S, R, 0, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    case 1: launch_after(face_flux_ops_kernel<S, R, 1, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    case 2: launch_after(face_flux_ops_kernel<S, R, 2, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    default: launch_after(face_flux_ops_kernel<S, R, 3, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
   }
 }
 
@@ -431,7 +434,7 @@ int launch_face_flux_ops(const S* pool, const PatchDesc* patches, const FaceFlux
 template <typename S>
 int launch_reflux_apply(S* pool, const PatchDesc* patches, const RefluxOp* ops, int nops, double* reg,
                         const double* dt, cudaStream_t stream) {
-  if (nops > 0) reflux_apply_kernel<S><<<nops, 128, 0, stream>>>(pool, patches, ops, reg, dt);
+  if (nops > 0) launch_after(reflux_apply_kernel<S>, nops, 128, 0, stream, pool, patches, ops, reg, dt);
   return check_launch("reflux");
 }
 

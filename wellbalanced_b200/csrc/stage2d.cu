@@ -91,6 +91,7 @@ struct Occupancy2D {
 // are float64.
 template <typename S, typename R, int LIM, bool PHYS, int TX, int TY>
 __global__ void __launch_bounds__(kThreads2D, (Occupancy2D<S, R>::kBlocks)) stage2d_kernel(const StageArgs<S> a) {
+  after_previous();
   using M = Math<R>;
   // phase 1 (cells -> primitive variables) in the state's type; a float64 state with
   // float32 arithmetic takes float32-seeded float64 reciprocals there
@@ -394,7 +395,7 @@ void launch_shape(const StageArgs<S>& args, int ntiles, cudaStream_t stream) {
   const size_t smem = sizeof(R) * (11 * NC + 14 * NF);
   cudaFuncSetAttribute(stage2d_kernel<S, R, LIM, PHYS, TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        int(smem));
-  stage2d_kernel<S, R, LIM, PHYS, TX, TY><<<ntiles, kThreads2D, smem, stream>>>(args);
+  launch_after(stage2d_kernel<S, R, LIM, PHYS, TX, TY>, ntiles, kThreads2D, smem, stream, args);
 }
 
 // One limiter: the default shape (ideal or non-ideal) or one of the other shapes (ideal).

@@ -146,6 +146,7 @@ __device__ __forceinline__ void yz_faces(const R* P, int NR, int ry, int sy, int
 template <typename S, typename R, int LIM, bool PHYS, int TY, int TZ>
 __global__ void __launch_bounds__(threads3d<TY, TZ>(), (Occupancy3D<R, PHYS, TY, TZ>::kBlocks))
     stage3d_kernel(const StageArgs<S> a) {
+  after_previous();
   using M = Math<R>;
   using W = S;  // phase A's arithmetic: the state's type
   using MW = typename std::conditional<std::is_same<S, R>::value, Math<S>, MathRefined>::type;
@@ -557,7 +558,7 @@ void launch_shape3d(const StageArgs<S>& args, int ntiles, cudaStream_t stream) {
   constexpr size_t smem = smem3d<R, PHYS, TY, TZ>();
   cudaFuncSetAttribute(stage3d_kernel<S, R, LIM, PHYS, TY, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        int(smem));
-  stage3d_kernel<S, R, LIM, PHYS, TY, TZ><<<ntiles, threads3d<TY, TZ>(), smem, stream>>>(args);
+  launch_after(stage3d_kernel<S, R, LIM, PHYS, TY, TZ>, ntiles, threads3d<TY, TZ>(), smem, stream, args);
 }
 
 template <typename S, typename R, int LIM>
