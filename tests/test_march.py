@@ -35,3 +35,23 @@ def test_merged_parts_share_one_march():
     assert merged.march == min(part.march for part in parts)
     for count in _covered(merged):
         assert np.all(count == 1)
+
+
+@pytest.mark.parametrize("precision", [32, 64, 6432])
+@pytest.mark.parametrize("shape", [(4, 4), (33, 17), (64, 64), (200, 31), (501, 339), (2000, 1500)])
+def test_the_suited_2d_tile_is_a_built_one_and_covers_the_patch(shape, precision):
+    from wellbalanced_b200 import _lib
+
+    layout = Layout(AMRHierarchy(shape, periodic=(True, False)), precision=precision)
+    tile = layout.suited_tile()
+    assert tile in _lib.tile_shapes(2, precision)
+    layout.set_tile(tile)
+    count = np.zeros(layout._extents()[0], dtype=int)
+    for t in layout.tiles:
+        count[int(t["x0"]) : int(t["x0"]) + tile[0], int(t["y0"]) : int(t["y0"]) + tile[1]] += 1
+    assert np.all(count == 1)
+
+
+def test_many_tiles_keep_the_default_shape():
+    layout = Layout(AMRHierarchy((4096, 4096), periodic=(True, True)), precision=32)
+    assert layout.suited_tile() == layout.default_tile

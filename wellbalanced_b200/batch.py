@@ -59,10 +59,11 @@ class Batch:
         self._auto_tile = tile == "auto"
         self.tile = None if tile is None or self._auto_tile else tuple(tile)
         self.tile_timings = None
-        if self.tile is not None:
+        tile = self.layout.suited_tile() if self.tile is None else self.tile
+        if tile != self.layout.tile_shape:
             from wellbalanced_b200.autotune import _set_tile
 
-            _set_tile(self.engine, self.tile)
+            _set_tile(self.engine, tile)
 
     @classmethod
     def orszag_tang(cls, count, *, seed=0, precision=32, **options):

@@ -56,7 +56,7 @@ class Engine:
     """Device pools + op lists of one hierarchy; the kernels' launch sequence."""
 
     def __init__(self, hierarchy, *, precision=32, walls=None, limiter=1, gamma=5.0 / 3.0, mean_field=(0.0, 0.0, 0.0),
-                 instances=None, device="cuda", lx=32, stream=None, layout=None):
+                 instances=None, device="cuda", lx=32, stream=None, layout=None, suit_tile=False):
         precision = _lib.precision_code(precision)
         if not torch.cuda.is_available():
             raise RuntimeError("wellbalanced_b200 needs a CUDA device (there is no CPU path)")
@@ -68,7 +68,7 @@ class Engine:
         self.gamma = float(gamma)
         self.mean_field = tuple(float(b) for b in mean_field) + (0.0,) * (3 - len(mean_field))
         self.layout = layout if layout is not None else Layout(
-            hierarchy, walls=walls, precision=precision, lx=lx, instances=instances)
+            hierarchy, walls=walls, precision=precision, lx=lx, instances=instances, suit_tile=suit_tile)
         L = self.layout
         self.ndim = L.ndim
         #: finest level of the layout (the hierarchy's property walks every patch)
@@ -178,7 +178,8 @@ class Engine:
 
     def __setattr__(self, name, value):
         object.__setattr__(self, name, value)
-        if name not in Engine._COUNTERS:  # another setting or buffer: the lists are out of date
+        # another setting or buffer: the lists are out of date
+        if name not in Engine._COUNTERS and self.__dict__.get("_lists"):
             object.__setattr__(self, "_lists", {})
 
     def _s(self):

@@ -385,7 +385,7 @@ class Layout:
     """Pool layout, work lists and op lists of a hierarchy for the MHD state."""
 
     def __init__(self, hierarchy: AMRHierarchy, *, walls=None, precision=32, lx=32, instances=None,
-                 align=8, tile=None):
+                 align=8, tile=None, suit_tile=False):
         self.h = hierarchy
         self.ndim = hierarchy.ndim
         if self.ndim not in (2, 3):
@@ -399,6 +399,8 @@ class Layout:
         self.exact_march = False
         #: 2D: the (tx, ty) tile shape of the stage kernel's work list (None: the default)
         self.tile = None if tile is None else tuple(int(v) for v in tile)
+        #: 2D without `tile`: cut for `suited_tile` instead of the default shape
+        self._suit_tile = suit_tile and self.ndim == 2
         self.walls = walls or ((False, False),) * self.ndim
         patches = hierarchy.patches
         self.npatches = len(patches)
@@ -554,6 +556,8 @@ class Layout:
             if self.tile not in _lib.tile_shapes(self.ndim, self.precision):
                 raise ValueError(f"no {self.tile} tile shape; built: {_lib.tile_shapes(self.ndim, self.precision)}")
             self.tile_shape = self.tile
+        elif self._suit_tile:
+            self.tile_shape = self.suited_tile()
         del lib
         self._cut_tiles()
 
@@ -571,6 +575,26 @@ class Layout:
         columns of `march` cell planes)."""
         self.march = self.lx if self.ndim == 2 or self.exact_march else self._short_march()
         self.tiles = self._tiles_of(self.march)
+
+    def suited_tile(self):
+        """The 2D tile shape that finishes earliest by a model of the stage kernel: an SM works
+        through tiles / SMs of them, each its faces, haloed cells and cells (weighed 1, 0.35 and
+        0.35) and 500 for its start and barriers; the last ones add their own latency, a round
+        of 256 faces about 900. The default unless another wins 3%. B200, a step on the default
+        -> on the choice: 64^2 float64 32.8 -> 26.2 us (8x16), 64^2 float32 30.8 -> 23.2 (8x32),
+        501 x 339 float32 49.4 -> 43.8 (8x32), the 865-patch sheet 214 -> 195 (16x16); 256^2
+        float64 keeps 8x32 (43.4; 8x16: 49.3), 700^2 float32 16x32 (86.6; 8x32: 91.1)."""
+        size = self._extents()
+        shapes = _lib.tile_shapes(2, self.precision)
+        best, cost = self.default_tile, None
+        for tx, ty in shapes:
+            tiles = int((-(-size[:, 0] // tx) * -(-size[:, 1] // ty)).sum())
+            faces = 2 * (tx + 1) * (ty + 1)
+            found = (tiles / SMS * (faces + 0.35 * ((tx + 4) * (ty + 4) + tx * ty) + 500.0)
+                     + 1300.0 + 900.0 * -(-faces // 256))
+            if cost is None or found < 0.97 * cost:
+                best, cost = (tx, ty), found
+        return best
 
     def _extents(self):
         """Cells and owned upper node planes of every patch (patches x axes)."""

@@ -138,16 +138,18 @@ class MHD2D:
                        mean_field=self.mean_field, device=self.device)
         from wellbalanced_b200.distributed import solver_engine, solver_group
 
+        physics = (self.resistivity, self.conduction[0], self.conduction[1], self.gravity[0], self.gravity[1])
         # a hierarchy over several ranks (AMRHierarchy(..., comm=group)): this rank's patches
         self._group = solver_group(self.hierarchy)
         if self._group is not None:
             self.engine = solver_engine(self.hierarchy, self._group, walls=walls, **options)
         else:
-            self.engine = Engine(self.hierarchy, walls=walls, **options)
+            # the tile shape by the grid's size; the non-ideal terms run on the default one
+            self.engine = Engine(self.hierarchy, walls=walls, **options,
+                                 suit_tile=self.tile is None and self._fused and not any(physics))
         groups = self.engine.layout.groups
         self._groups_all = groups
         self._groups_potential = groups[1:]
-        physics = (self.resistivity, self.conduction[0], self.conduction[1], self.gravity[0], self.gravity[1])
         if any(physics):
             self.engine.physics = tuple(float(v) for v in physics)
         # the conduction limit depends on the density: on a refined hierarchy each level's
