@@ -89,48 +89,63 @@ __device__ __forceinline__ void copy_op(S* __restrict__ pool, const PatchDesc* _
   }
 }
 
-// The points of one copy op, two per thread and pass (the loads of both, every field,
-// before the stores; an op never writes a point it reads): for the standalone copy
-// launches, whose ops are large where the lists are (a big box's halos).
+// A plain copy (w1 = 1, no second source, nothing negated) of NF fields of up to two points:
+// all loads before the stores.
+template <typename S, int NF>
+__device__ __forceinline__ void copy_two(S* __restrict__ pool, bool both, int64_t d0, int64_t d1, int64_t fd, int64_t s0,
+                                         int64_t s1, int64_t fs) {
+  S v[2][NF];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    v[0][f] = pool[s0 + f * fs];
+    if (both) v[1][f] = pool[s1 + f * fs];
+  }
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    pool[d0 + f * fd] = v[0][f];
+    if (both) pool[d1 + f * fd] = v[1][f];
+  }
+}
+
+// The points of one copy op, two per thread and pass where it is a plain copy (an op never
+// writes a point it reads): for the standalone copy launches, whose ops are large where the
+// lists are (a big box's halos). Other copies go as copy_op. B200, a fill: 256^3 float32 54 ->
+// 45 us, 150 x 97 x 75 float64 17.1 -> 13.8 us, 512 planes 53 -> 34 us.
 template <typename S, int NT = kOpThreads>
 __device__ __forceinline__ void copy_op_pairs(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
                                               const CopyOp& op) {
-  const PatchDesc D = patches[op.dst];
-  const PatchDesc A = patches[op.src1];
-  const PatchDesc B = patches[op.src2 >= 0 ? op.src2 : op.src1];
+  const int nf = op.field_hi - op.field_lo;
+  if (!(op.w1 == 1.0 && op.w2 == 0.0 && op.negate < 0) || (nf != 1 && nf != 5 && nf != 6)) {
+    copy_op<S, NT>(pool, patches, op);
+    return;
+  }
+  const PatchDesc& D = patches[op.dst];
+  const PatchDesc& A = patches[op.src1];
+  const int64_t fd = D.fstride, fs = A.fstride;
+  const int64_t bd = D.off + op.field_lo * fd, bs = A.off + op.field_lo * fs;
+  const int64_t dp0 = D.pitch0, dp1 = D.pitch1, sp0 = A.pitch0, sp1 = A.pitch1;
   // 32-bit point index (the host keeps every op below 2^31 points)
   const unsigned n1 = unsigned(op.n[1]), n2 = unsigned(op.n[2]);
   const unsigned count = unsigned(op.n[0]) * n1 * n2;
   for (unsigned t0 = op_lane<NT>(); t0 < count; t0 += 2 * NT) {
-    S v[2][8];
-    int64_t od[2];
+    int64_t d[2], s[2];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-      const unsigned t = t0 + u * NT;
-      if (t >= count) continue;
+      const unsigned t = min(t0 + u * NT, count - 1);
       const unsigned line = t / n2;
       const int p2 = int(t - line * n2);
-      const int p1 = int(line % n1);
       const int p0 = int(line / n1);
-      od[u] = offset_of(D, op.d[0] + p0, op.d[1] + p1, op.d[2] + p2);
-      const int64_t o1 = offset_of(A, op.s1[0] + op.m1[0] * p0, op.s1[1] + op.m1[1] * p1, op.s1[2] + op.m1[2] * p2);
-      const int64_t o2 = offset_of(B, op.s2[0] + op.m2[0] * p0, op.s2[1] + op.m2[1] * p1, op.s2[2] + op.m2[2] * p2);
-#pragma unroll
-      for (int f = 0; f < 8; ++f) {
-        if (f >= op.field_lo && f < op.field_hi) {
-          S x = S(op.w1) * pool[A.off + f * A.fstride + o1];
-          if (op.w2 != 0.0) x += S(op.w2) * pool[B.off + f * B.fstride + o2];
-          v[u][f] = f == op.negate ? -x : x;
-        }
-      }
+      const int p1 = int(line - unsigned(p0) * n1);
+      d[u] = bd + pitched(dp0, dp1, op.d[0] + p0, op.d[1] + p1, op.d[2] + p2);
+      s[u] = bs + pitched(sp0, sp1, op.s1[0] + op.m1[0] * p0, op.s1[1] + op.m1[1] * p1, op.s1[2] + op.m1[2] * p2);
     }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (t0 + u * NT >= count) continue;
-#pragma unroll
-      for (int f = 0; f < 8; ++f)
-        if (f >= op.field_lo && f < op.field_hi) pool[D.off + f * D.fstride + od[u]] = v[u][f];
-    }
+    const bool both = t0 + NT < count;
+    if (nf == 1)
+      copy_two<S, 1>(pool, both, d[0], d[1], fd, s[0], s[1], fs);
+    else if (nf == 5)
+      copy_two<S, 5>(pool, both, d[0], d[1], fd, s[0], s[1], fs);
+    else
+      copy_two<S, 6>(pool, both, d[0], d[1], fd, s[0], s[1], fs);
   }
 }
 
