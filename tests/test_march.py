@@ -21,9 +21,11 @@ def _covered(layout):
 
 @pytest.mark.parametrize("shape", [(4, 4, 4), (7, 5, 33), (64, 64, 64), (150, 97, 75), (256, 256, 256)])
 @pytest.mark.parametrize("lx", [3, 5, 32])
-def test_every_cell_lies_in_one_tile(shape, lx):
-    layout = Layout(AMRHierarchy(shape, periodic=(True, False, True)), precision=32, lx=lx)
+@pytest.mark.parametrize("precision, suit", [(32, False), (32, True), (64, True), (6432, True)])
+def test_every_cell_lies_in_one_tile(shape, lx, precision, suit):
+    layout = Layout(AMRHierarchy(shape, periodic=(True, False, True)), precision=precision, lx=lx, suit_tile=suit)
     assert 1 <= layout.march <= lx
+    assert suit or layout.tile_shape == layout.default_tile
     for count in _covered(layout):
         assert np.all(count == 1)
 

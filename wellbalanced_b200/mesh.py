@@ -399,8 +399,8 @@ class Layout:
         self.exact_march = False
         #: 2D: the (tx, ty) tile shape of the stage kernel's work list (None: the default)
         self.tile = None if tile is None else tuple(int(v) for v in tile)
-        #: 2D without `tile`: cut for `suited_tile` instead of the default shape
-        self._suit_tile = suit_tile and self.ndim == 2
+        #: without `tile`: cut for the shape that suits the grid instead of the default one
+        self._suit_tile = suit_tile
         self.walls = walls or ((False, False),) * self.ndim
         patches = hierarchy.patches
         self.npatches = len(patches)
@@ -556,8 +556,6 @@ class Layout:
             if self.tile not in _lib.tile_shapes(self.ndim, self.precision):
                 raise ValueError(f"no {self.tile} tile shape; built: {_lib.tile_shapes(self.ndim, self.precision)}")
             self.tile_shape = self.tile
-        elif self._suit_tile:
-            self.tile_shape = self.suited_tile()
         del lib
         self._cut_tiles()
 
@@ -573,7 +571,15 @@ class Layout:
     def _cut_tiles(self):
         """The stage kernel's work list: every patch's computed cells and nodes in tiles (3D:
         columns of `march` cell planes)."""
-        self.march = self.lx if self.ndim == 2 or self.exact_march else self._short_march()
+        suit = self._suit_tile and self.tile is None
+        self.march = self.lx
+        if self.ndim == 2:
+            if suit:
+                self.tile_shape = self.suited_tile()
+        elif not self.exact_march:
+            # 16 x 32 tiles (float32) are the autotuner's: one CTA an SM
+            shapes = _lib.tile_shapes(3, self.precision)[:2] if suit else [self.tile_shape]
+            self.tile_shape, self.march = self._suited_march(shapes)
         self.tiles = self._tiles_of(self.march)
 
     def suited_tile(self):
@@ -609,30 +615,40 @@ class Layout:
                  for origin in itertools.product(*(range(0, n, step) for n, step in zip(size, steps, strict=True)))]
         return np.array(tiles, dtype=np.int32).view(_lib.TILE).reshape(-1) if tiles else np.zeros(0, _lib.TILE)
 
-    def _short_march(self):
-        """Cell planes per tile: `lx`, or the halving of it (4 at least) that finishes earliest
-        where few columns leave SMs idle. A tile of L planes costs about L + 2.5 (its first
-        planes are loads and half the faces only), and an SM works through ceil(tiles / SMs) of
-        them, the longest among them; a shorter march has to win 2%. B200, before -> after:
-        64^3 float64 (16 columns) 389 -> 123 us a launch at 8 planes, 150 x 97 x 75 mixed
-        303 -> 259 us at 8, the 203-patch 64^3 multi-blast 269 -> 157 us at 8; 256^3 keeps 32
-        (2014 us; 16: 2104, 8: 2312)."""
+    #: (latency of a plane of a tile that has its SM to itself, its share of a busy SM's time,
+    #: planes' worth of work before the first full one) of the 3D tiles by their columns along
+    #: y, for float32 and float64 faces: fitted to 80 stage launches of 32^3 to 256^3 boxes on a
+    #: B200 (8% rms in float32, 16% in float64; the choice at most 2% off the best measured)
+    _PLANE_COSTS = {False: {16: (1.0, 0.78, 2.5), 8: (0.73, 0.33, 3.7)}, True: {16: (1.0, 1.17, 3.0), 8: (0.94, 0.66, 1.35)}}
+
+    def _suited_march(self, shapes):
+        """(tile shape, cell planes per tile): of `shapes` and of `lx` and its halvings (4 at
+        least) the pair that finishes earliest, where few columns leave SMs idle: a tile's own
+        planes, then the SM's other tiles. The first shape and `lx` stand unless another pair
+        wins 2%, and where they give every SM more than eight tiles. B200, a stage launch with 16 x
+        16 tiles of 32 planes -> the choice: 64^3 float64 357 -> 108 us (8 planes), 32^3 float32
+        165 -> 28 (8 x 16, 4 planes), 150 x 97 x 75 mixed 310 -> 203 (8 x 16, 16), the 203-patch
+        64^3 multi-blast 255 -> 137 (8 x 16, 8); 256^3 float32 keeps them (1789 us; 8 x 16: 1817,
+        16 planes: 1882)."""
         size = self._extents()
+        best, cost = (shapes[0], self.lx), None
         if size.size == 0:
-            return self.lx
-        a, b = self.tile_shape
-        columns = -(-size[:, 1] // a) * -(-size[:, 2] // b)
-        best, cost = self.lx, None
-        march = self.lx
-        while march >= 4 or march == self.lx:
-            tiles = -(-size[:, 0] // march)
-            count = int((tiles * columns).sum())
-            planes = float((columns * (size[:, 0] + 2.5 * tiles)).sum()) / count
-            longest = min(march, int(size[:, 0].max())) + 2.5
-            found = longest + (-(-count // SMS) - 1) * planes
-            if cost is None or found < 0.98 * cost:
-                best, cost = march, found
-            march //= 2
+            return best
+        costs = self._PLANE_COSTS[self.precision == 64]
+        for a, b in shapes:
+            latency, share, start = costs[a]
+            columns = -(-size[:, 1] // a) * -(-size[:, 2] // b)
+            march = self.lx
+            while march >= 4 or march == self.lx:
+                tiles = -(-size[:, 0] // march)
+                count = int((tiles * columns).sum())
+                planes = float((columns * (size[:, 0] + start * tiles)).sum()) / count
+                found = (min(march, int(size[:, 0].max())) + start) * latency + max(0.0, count / SMS - 1.0) * planes * share
+                if cost is None and count > 8 * SMS:
+                    return best
+                if cost is None or found < 0.98 * cost:
+                    best, cost = ((a, b), march), found
+                march //= 2
         return best
 
     def _chunks(self, per=2048):
@@ -954,6 +970,7 @@ class Layout:
         out.march = min(part.march for part in layouts)
         out.wraps = all(part.wraps for part in layouts)
         out.exact_march = True
+        out._suit_tile = False
         rows, tiles, chunk_patch, chunk_start, inv, inv_levels = [], [], [], [], [], []
         same_levels, boundary_levels, interp_levels = {}, {}, {}
         restrict_levels, face_ops = {}, []

@@ -106,16 +106,17 @@ class MHD3D:
                        mean_field=self.mean_field, device=self.device)
         from wellbalanced_b200.distributed import solver_engine, solver_group
 
+        physics = (self.resistivity, *self.gravity)
         # a hierarchy over several ranks (AMRHierarchy(..., comm=group)): this rank's patches
         self._group = solver_group(self.hierarchy)
         if self._group is not None:
             self.engine = solver_engine(self.hierarchy, self._group, lx=self.lx, **options)
         else:
-            self.engine = Engine(self.hierarchy, lx=self.lx, **options)
+            # the tile shape by the grid's size; the non-ideal terms run on the default one
+            self.engine = Engine(self.hierarchy, lx=self.lx, **options, suit_tile=self._fused and not any(physics))
         groups = self.engine.layout.groups
         self._groups_all = groups
         self._groups_potential = groups[1:]
-        physics = (self.resistivity, *self.gravity)
         if any(physics):
             self.engine.physics = tuple(float(v) for v in physics)
 
