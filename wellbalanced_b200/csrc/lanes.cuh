@@ -6,10 +6,13 @@
 // mask `M2`; selects, min / max, absolute values and the special functions act on each
 // lane.
 //
-// `L1` is one float32 lane with the same rounding: every add, subtract and multiply is
-// rounded on its own (no implicit contraction into FMA) and every fused multiply-add is
-// written as `fma`, so a value has the same bits in a lane of F2 and in L1, and the
-// kernels that form the same face (the stage kernels, the refluxing kernel) agree on it.
+// `L1` is one float32 lane: every add, subtract and multiply is rounded on its own and
+// every fused multiply-add is written as `fma`. The assembler, however, joins a packed
+// multiply and the packed add that alone reads it into one packed fma, whatever rounding
+// they are written with, so an F2 value keeps its bits only while the operations around it
+// stay as they are; where a product must be rounded, `lproduct` forms it lane by lane. The
+// kernels that form the same face (the stage kernels, the refluxing kernel) run the same
+// lane code and agree on its bits.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -18,7 +18,8 @@ namespace wb {
 // selects, compares and min / max (half the rate of the multiply-adds): the forms below are
 // chosen for few of those, each with the bits of the plain selection. Per face: 57 fewer than
 // selecting every variant (limiter 14, square roots 6, first-order fallback 12, star states
-// 10, sign 3, region selection 12).
+// 10, sign 3, region selection 12). B200: a stage of the 256^3 box 1.98 ms with those, 1.77
+// now; of 512 2D instances of 32^2 to 256^2 cells, 0.90 and 0.81 ms.
 
 // sqrt(x) as x rsqrt(x); x below the smallest normal (zero and negative discriminants) counts
 // as that, so the root of zero is 1e-19: far under the rounding of what it is added to.

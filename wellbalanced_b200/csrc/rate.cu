@@ -102,7 +102,10 @@ int launch_finalize_dt(const unsigned long long* keys, int ninstances, double cf
 // where it would change the key), and the last block to finish turns the keys into every
 // instance's dt, hands them on in `keys` / `level_keys` and puts the scratch back to the
 // identities for the next launch. Three launches (keys, rate, dt) and 8 serial rounds a block
-// before; small grids, whose few chunks left most SMs idle, take 8 blocks a chunk.
+// before; small grids, whose few chunks left most SMs idle, take 8 blocks a chunk. B200, the
+// three launches and this one: a 32^2 float64 grid 9.7 and 6.0 us, 256^2 14.2 and 7.2, a 256^3
+// float32 box 194 and 162, 512 2D float32 instances 95 and 98 (bound by the reads of the state
+// and the latency of the chain behind them; the batch's blocks by their look-ups).
 struct StableDt {
   double cfl, eta, kappa, gamma;
   const double *inv_dx2_sum, *inv_dx2_levels;
