@@ -8,7 +8,9 @@ through the C ABI:
   level: interpolation from the level below, same-level copies, outflow / wall faces;
 * ``restrict(pool, groups)`` — patchwork's ``restrict``;
 * ``stage(...)`` — one fused RK stage over every tile;
-* ``rate()`` / ``finalize_dt()`` — the stable step on the device.
+* ``stable_dt()`` — the stable step on the device in one launch (``rate()`` and
+  ``finalize_dt()`` apart where ranks reduce between them);
+* ``run_steps(...)`` — whole steps from a launch list put together once.
 
 One step is the reference's ``step`` (``carafe/mhd.py:965-994``,
 ``carafe/mhd3d.py:726-754``): stage 1 into U1, restrict the potential, fill U1, stage 2
