@@ -165,8 +165,8 @@ class Engine:
         self._lists = {}
         #: run the reflux, restriction, halo-fill and stable-step phases between the stage
         #: kernels as op programs (`wb_run_program`, one launch each: six launches per
-        #: refined step instead of ~26). Off by default: on the B200 the separate launches
-        #: finish the ~2300-patch Harris step in 0.62 ms against 0.74 ms for the programs,
+        #: refined step instead of 24). Off by default: on the B200 the separate launches
+        #: finish the ~2300-patch Harris step in 0.38 ms against 0.51 ms for the programs,
         #: whose in-kernel phase waits cost more than the launch boundaries they replace
         self.use_programs = False
         self._programs = {}
@@ -183,6 +183,19 @@ class Engine:
         # another setting or buffer: the lists are out of date
         if name not in Engine._COUNTERS and self.__dict__.get("_lists"):
             object.__setattr__(self, "_lists", {})
+        if name == "physics" and value is not None:
+            self._default_tiles()
+
+    def _default_tiles(self):
+        """The non-ideal kernels run on the default tile: a work list cut to a shape chosen by
+        the grid's size (not one asked for) is cut again."""
+        layout = self.layout
+        if getattr(layout, "_suit_tile", False) and layout.tile is None and layout.tile_shape != layout.default_tile:
+            layout._suit_tile = False
+            layout.tile_shape = layout.default_tile
+            layout._cut_tiles()
+            self.tiles = _device_bytes(layout.tiles, self.device, _lib.TILE)
+            self.ntiles = int(layout.tiles.size)
 
     def _s(self):
         if self._step_stream is not None:
