@@ -18,6 +18,10 @@
  *     a device work list of patch tiles, the per-step rate / dt reduction, and the
  *     halo / restriction / flux-register op lists. Structs are laid out as in
  *     wellbalanced_b200/csrc/layout.cuh and halo.cuh (mirrored by the Python host).
+ *     The launches of a step overlap with the kernel before them in their stream and wait
+ *     for it before they read a state, a dt or a flux buffer. The tables (patches, tiles,
+ *     work lists, ops) may be read ahead of that wait: a caller that fills them with a
+ *     kernel of its own waits for it; copies to the device need nothing.
  */
 #ifndef WELLBALANCED_B200_H
 #define WELLBALANCED_B200_H

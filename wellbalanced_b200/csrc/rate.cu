@@ -118,7 +118,7 @@ struct StableDt {
 
 // (float32: 32 registers, 64 warps an SM, as the rate kernel alone)
 template <typename S, int NDIM>
-__global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4) stable_dt_kernel(const S* __restrict__ pool, const PatchDesc* patches,
+__global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4) stable_dt_kernel(const S* pool, const PatchDesc* patches,
                                                                  const int* chunk_patch, const int* chunk_start,
                                                                  int nchunks, int parts, double b0x, double b0y,
                                                                  double b0z, const RateSlots scratch,

@@ -276,7 +276,7 @@ constexpr int kFluxWarps = kFluxThreads / 32;
 inline int flux_splits(int nops) { return max(1, min(32, 148 * 64 / max(nops, 1))); }
 
 template <typename S, typename R, int LIM, bool PHYS>
-__global__ void __launch_bounds__(kFluxThreads) face_flux_ops_kernel(const S* __restrict__ pool,
+__global__ void __launch_bounds__(kFluxThreads) face_flux_ops_kernel(const S* pool,
                                                                      const PatchDesc* __restrict__ patches,
                                                                      const FaceFluxOp* __restrict__ ops, int nops,
                                                                      int splits, double b0x, double b0y, double b0z, double gamma,
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kFluxThreads) face_flux_ops_kernel(const S* __
 template <typename S>
 __global__ void reflux_apply_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
                                     const RefluxOp* __restrict__ ops, double* __restrict__ reg,
-                                    const double* __restrict__ dt) {
+                                    const double* dt) {
   after_previous();
   reflux_op<S, 128>(pool, patches, ops[blockIdx.x], reg, dt);
 }
@@ -344,8 +344,8 @@ constexpr int kStagedThreads = 128;
 
 template <typename S, typename R, int LIM>
 __global__ void __launch_bounds__(kStagedThreads) face_flux_staged_kernel(
-    const S* __restrict__ pool, const PatchDesc* __restrict__ patches, const FaceFluxOp* __restrict__ ops, int nops,
-    int nfaces, double b0x, double b0y, double b0z, double gamma, const double* __restrict__ bflux,
+    const S* pool, const PatchDesc* __restrict__ patches, const FaceFluxOp* __restrict__ ops, int nops, int nfaces,
+    double b0x, double b0y, double b0z, double gamma, const double* bflux,
     double* __restrict__ reg) {
   after_previous();
   const int face = blockIdx.x * kStagedThreads + threadIdx.x;

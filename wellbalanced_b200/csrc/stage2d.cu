@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kThreads2D, (Occupancy2D<S, R>::kBlocks)) stag
   const PatchDesc P = a.patches[tile.patch];
   const int nx = P.n[0], ny = P.n[1];
   const int64_t pitch = P.pitch0, fs = P.fstride;
-  const S* __restrict__ src = a.src + P.off;
+  const S* src = a.src + P.off;
   const R dx = R(P.dx[0]), dy = R(P.dx[1]);
   const R idx = M::inv(dx), idy = M::inv(dy);
   const R gamma = R(a.gamma), inv_gm1 = R(a.inv_gm1);
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(kThreads2D, (Occupancy2D<S, R>::kBlocks)) stag
   const S dt = S(a.dt[P.instance]);
   // the inverse spacings of the float64 flux differences (mixed precision only)
   const S sidx = kMixed ? S(1) / S(P.dx[0]) : S(0), sidy = kMixed ? S(1) / S(P.dx[1]) : S(0);
-  const S* __restrict__ base_state = a.base ? a.base + P.off : nullptr;
+  const S* base_state = a.base ? a.base + P.off : nullptr;
   S* __restrict__ dst = a.dst + P.off;
   constexpr int NIT = (TX * TY + kThreads2D - 1) / kThreads2D;  // phase-3 rounds of the threads
   S in_cell[NIT][6], in_node[NIT], base_cell[NIT][6], base_node[NIT];

@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(threads3d<TY, TZ>(), (Occupancy3D<R, PHYS, TY,
   const PatchDesc P = a.patches[tile.patch];
   const int nx = P.n[0], ny = P.n[1], nz = P.n[2];
   const int64_t p0 = P.pitch0, p1 = P.pitch1, fs = P.fstride;
-  const S* __restrict__ src = a.src + P.off;
+  const S* src = a.src + P.off;
   const R dx = R(P.dx[0]), dy = R(P.dx[1]), dz = R(P.dx[2]);
   const R idx = M::inv(dx), idy = M::inv(dy), idz = M::inv(dz);
   const R gamma = R(a.gamma), inv_gm1 = R(a.inv_gm1);
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(threads3d<TY, TZ>(), (Occupancy3D<R, PHYS, TY,
            M::div(face(plane, 0, j, k) - face(plane, 0, j - 1, k), dy, idy);
   };
   const S dt = S(a.dt[P.instance]);
-  const S* __restrict__ base_state = a.base ? a.base + P.off : nullptr;
+  const S* base_state = a.base ? a.base + P.off : nullptr;
   S* __restrict__ dst = a.dst + P.off;
   unsigned bad = 0;
   // phase A's spacings and mean field in the state's type

@@ -34,7 +34,11 @@ inline int check_launch(const char* what) {
 // (programmatic stream serialization), each starts with `after_previous`, which waits until
 // the kernel before it in the stream has finished and its memory is visible, and then lets
 // the next one be set up. No kernel reads or writes global memory before that call, so the
-// order of all accesses is that of plain launches. B200: the refined sheet (25 launches a step)
+// order of all accesses is that of plain launches. That holds for coherent loads only: the
+// compiler may read what a `const T* __restrict__` kernel parameter points to through the
+// read-only path, or before the call, and the kernel before may still be writing it. So such
+// a parameter is for tables that no launch writes (patches, op lists); the pools, the dt, the
+// flux register and the boundary fluxes are not marked so. B200: the refined sheet (25 launches a step)
 // 542 -> 476 us for two steps, 256^2 float64 (3 a step) 214 -> 200 us for four.
 template <typename... P, typename... A>
 inline void launch_after(void (*kernel)(P...), int64_t grid, int threads, size_t smem, cudaStream_t stream, A... args) {
