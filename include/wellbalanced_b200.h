@@ -174,7 +174,9 @@ int wb_finalize_dt(const unsigned long long* keys, int ninstances, double cfl, d
  * level_keys and dt. scratch: 1 + 2 ninstances (+ ninstances nlevels) 64-bit words, a ticket
  * (0) and the identities of the keys (per instance 0x8000000000000000, 0xfff0000000000000;
  * per level 0xfff0000000000000); every launch leaves it so. Launches that share a scratch
- * must not overlap. */
+ * must not overlap: of two that do (with the same work list) either may form its dt from a
+ * part of the cells, as when wb_rate runs twice on one key buffer at a time; the scratch is
+ * as it should be once both have finished. */
 int wb_stable_dt(int precision, int ndim, const void* state, const void* patches, const int* chunk_patch,
                  const int* chunk_start, int nchunks, double b0x, double b0y, double b0z, double gamma,
                  unsigned long long* keys, int ninstances, unsigned long long* level_keys, int nlevels, double cfl,

@@ -81,3 +81,21 @@ def test_one_launch_equals_rate_and_dt(name, precision):
         for got, want in zip((engine.keys, engine.dt, engine.time, engine.level_keys), expect):
             assert torch.equal(got, want)
         assert torch.equal(engine.dt_scratch, scratch)
+
+
+def test_overlapping_launches_leave_the_scratch_whole():
+    """Stable steps of one engine on two streams at once may spoil each other's dt, never a
+    later one: the ticket and the keys are back at their start once both are done."""
+    engine = _plane((700, 500), 32)
+    engine.stable_dt(0.4)
+    torch.cuda.synchronize()
+    expect, scratch = engine.dt.clone(), engine.dt_scratch.clone()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(200):
+        for stream in streams:
+            with torch.cuda.stream(stream):
+                engine.stable_dt(0.4)
+    torch.cuda.synchronize()
+    assert torch.equal(engine.dt_scratch, scratch)
+    engine.stable_dt(0.4)
+    assert torch.equal(engine.dt, expect)

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4) stable_d
                                                                  const int* chunk_patch, const int* chunk_start,
                                                                  int nchunks, int parts, double b0x, double b0y,
                                                                  double b0z, const RateSlots scratch,
-                                                                 unsigned long long* ticket, const StableDt a) {
+                                                                 unsigned* ticket, const StableDt a) {
   after_previous();
   __shared__ double s_largest[kRateThreads / 32], s_smallest[kRateThreads / 32];
   __shared__ bool s_last;
@@ -164,7 +164,9 @@ __global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4) stable_d
   }
   if (threadIdx.x == 0) {
     __threadfence();  // the block's keys before its ticket
-    s_last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
+    // counts to the grid's size and wraps to zero by itself: two launches that overlap spoil
+    // their own dt, and the scratch is whole again when both have finished
+    s_last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
   }
   __syncthreads();
   if (!s_last) return;
@@ -183,7 +185,6 @@ __global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4) stable_d
     finalize_dt_one(i, a.keys, a.cfl, a.eta, a.kappa, a.gamma, a.inv_dx2_sum, a.level_keys, a.inv_dx2_levels, nlevels,
                     a.time, a.end, a.dt, a.advance);
   }
-  if (threadIdx.x == 0) *ticket = 0;
 }
 
 // scratch: 1 + 2 ninstances (+ ninstances nlevels) words: the ticket (0), then (key(0),
@@ -196,6 +197,7 @@ int launch_stable_dt(const S* state, const PatchDesc* patches, int ndim, const i
                      double* dt, int advance, unsigned long long* scratch, cudaStream_t stream) {
   const RateSlots slots{scratch + 1, ninstances, level_keys ? scratch + 1 + 2 * ninstances : nullptr, nlevels, nullptr};
   const StableDt a{cfl, eta, kappa, gamma, inv_dx2_sum, inv_dx2_levels, time, end, dt, advance, keys, level_keys};
+  unsigned* ticket = reinterpret_cast<unsigned*>(scratch);
   // up to 8 blocks a chunk while they make at most 4 blocks an SM: a block costs ~3 us besides
   // its cells (work-list look-up, reduction, ticket), which more rounds carry better
   int parts = 8;
@@ -203,10 +205,10 @@ int launch_stable_dt(const S* state, const PatchDesc* patches, int ndim, const i
   const int grid = max(nchunks * parts, 1);
   if (ndim == 2)
     launch_after(stable_dt_kernel<S, 2>, grid, kRateThreads, 0, stream, state, patches, chunk_patch, chunk_start, nchunks, parts,
-                                                             b0[0], b0[1], b0[2], slots, scratch, a);
+                                                             b0[0], b0[1], b0[2], slots, ticket, a);
   else
     launch_after(stable_dt_kernel<S, 3>, grid, kRateThreads, 0, stream, state, patches, chunk_patch, chunk_start, nchunks, parts,
-                                                             b0[0], b0[1], b0[2], slots, scratch, a);
+                                                             b0[0], b0[1], b0[2], slots, ticket, a);
   return check_launch("stable_dt");
 }
 

@@ -344,7 +344,8 @@ class Engine:
         self.launches += 1
 
     def stable_dt(self, cfl, eta=0.0, kappa=0.0, *, advance=False):
-        """`rate` of the state and `finalize_dt` in one launch."""
+        """`rate` of the state and `finalize_dt` in one launch (as for them, one stream at a time:
+        the keys and the dt are the engine's own)."""
         b = self.mean_field
         levels = self.per_level_dt
         self._launch("wb_stable_dt", self.precision, self.ndim, self.state.data_ptr(), self.patches.data_ptr(),
