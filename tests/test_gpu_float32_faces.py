@@ -1,0 +1,91 @@
+"""float32 faces at their edges (GPU): no star state on a cold supersonic face, vanishing
+normal fields and star denominators, slopes of either sign and none, against float64 faces."""
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+def _uniform(ndim, axis, speed, pressure, precision):
+    """A uniform flow along `axis` (density 1, no field) set by its conserved values."""
+    from wellbalanced_b200 import MHD2D, MHD3D
+    from wellbalanced_b200.mesh import AMRHierarchy
+
+    shape = (20, 12, 9)[:ndim]
+    mesh = AMRHierarchy(shape, periodic=(True,) * ndim)
+    model = (MHD2D if ndim == 2 else MHD3D)(mesh, precision=precision, limiter="mc")
+    cells = [np.ones(shape)] + [np.full(shape, speed if a == axis else 0.0) for a in range(3)]
+    cells.append(np.full(shape, 1.5 * pressure + 0.5 * speed**2))
+    if ndim == 2:
+        model.set_conserved([*cells, np.zeros(shape)], np.zeros((21, 13)))
+    else:
+        nodes = [tuple(n + (a != c) for a, n in enumerate(shape)) for c in range(3)]
+        model.set_conserved(cells, [np.zeros(n) for n in nodes])
+    return model
+
+
+@pytest.mark.parametrize("ndim, axis", [(2, 0), (2, 1), (3, 0), (3, 1), (3, 2)])
+@pytest.mark.parametrize("sign", [1.0, -1.0])
+def test_a_cold_flow_keeps_the_upwind_flux(ndim, axis, sign):
+    """The fast speed (1.8e-7) is below half the spacing of float32 numbers at the velocity, so
+    S = S_M and no star state exists; the flux differences of the uniform flow are exact zeros."""
+    model = _uniform(ndim, axis, sign * 4.125, 2e-14, "mixed")
+    before = model.engine.state.clone()
+    model.step()
+    assert torch.equal(model.engine.state, before)
+
+
+@pytest.mark.parametrize("ndim, axis", [(2, 0), (2, 1), (3, 0), (3, 1), (3, 2)])
+def test_a_flow_without_pressure_stays_finite(ndim, axis):
+    model = _uniform(ndim, axis, 1.0, 0.0, 32)
+    before = model.engine.state.clone()
+    model.advance(1, check=False)
+    assert int(model.engine.bad.item()) > 0  # no valid state, and counted as that
+    assert torch.equal(model.engine.state, before)
+
+
+@pytest.mark.parametrize("limiter", ["minmod", "vanleer", "mc"])
+@pytest.mark.parametrize("speed", [0.3, 4.0])
+@pytest.mark.parametrize("field", ["none", "normal", "across", "out"])
+def test_faces_agree_with_float64(field, speed, limiter):
+    """Random cells with constant stripes (slopes of both signs, and zero) under a field that is
+    absent, along x (B_n = 0 on the y-faces, a vanishing star denominator on the x-faces, whose
+    fast speed is the Alfven speed), along y, or along z (B_n = 0 everywhere).
+
+    Bound: a float32 flux is good to 2e-3 of its scale (star denominators are used down to 1e-3
+    of their terms, with 1e-6 of rounding in them), four faces change a cell by dt / dx = 0.02 of
+    their errors each; the scale of a flux is the largest conserved value times the largest
+    signal speed."""
+    from wellbalanced_b200 import MHD2D
+    from wellbalanced_b200.mesh import AMRHierarchy
+
+    shape, ratio = (24, 40), 0.02
+    rng = np.random.default_rng(5)
+    stripes = (np.arange(shape[0]) // 4 % 3 == 0)[:, None]
+    draw = lambda lo, hi: np.where(stripes, 0.5 * (lo + hi), rng.uniform(lo, hi, shape))  # noqa: E731
+    rho, p = draw(0.6, 1.4), draw(0.6, 1.4)
+    velocity = [draw(-speed, speed) for _ in range(3)]
+    mean, bz = {"none": ((0.0, 0.0), 0.0), "normal": ((2.0, 0.0), 0.0), "across": ((0.0, -2.0), 0.0),
+                "out": ((0.0, 0.0), 1.5)}[field]
+    b2 = mean[0] ** 2 + mean[1] ** 2 + bz**2
+    energy = 1.5 * p + 0.5 * rho * sum(v * v for v in velocity) + 0.5 * b2
+    results = []
+    for precision in (64, "mixed"):
+        mesh = AMRHierarchy(shape, ((0.0, 0.6), (0.0, 1.0)), periodic=(True, True))
+        model = MHD2D(mesh, precision=precision, limiter=limiter, mean_field=mean)
+        model.set_conserved([rho, *(rho * v for v in velocity), energy, np.full(shape, bz)], np.zeros((25, 41)))
+        eng = model.engine
+        eng.dt.fill_(ratio * 0.025)
+        eng.bad.zero_()
+        eng.stage(eng.state, None, eng.stage_pool)
+        assert int(eng.bad.item()) == 0
+        (patch,) = mesh.patches
+        results.append([model._read(patch, f, node=f == 6, pool=eng.stage_pool).cpu().numpy() for f in range(7)])
+    signal = speed + np.sqrt((5.0 / 3.0 * 1.4 + b2) / 0.6)
+    bound = 4 * ratio * 2e-3 * float(np.abs(energy).max()) * signal
+    for want, got in zip(*results, strict=True):
+        assert np.isfinite(got).all()
+        assert np.abs(got - want).max() <= bound
