@@ -90,3 +90,17 @@ def test_a_bad_cell_is_counted_in_the_step_that_meets_it():
     model = _refined(2, precision=32)
     model.engine.bad.fill_(7)  # of an earlier call: each step counts its own
     model.step()
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+def test_a_cfl_of_its_own_each_step_takes_one_list(ndim):
+    listed, single = _refined(ndim, precision=32), _refined(ndim, precision=32)
+    for k in range(6):
+        for model in (listed, single):
+            model.cfl = 0.3 - 0.02 * k
+        listed.advance(1)
+        _one_by_one(single, 1)
+        assert len(listed.engine._lists) == 1
+        torch.cuda.synchronize()
+        assert torch.equal(listed.engine.state, single.engine.state)
+        assert torch.equal(listed.engine.status[1:], single.engine.status[1:])

@@ -22,6 +22,17 @@ def test_slots_hold_integers_pointers_and_double_bits():
         assert slot.view(np.float64) == 0.5 + k if t is _lib.c_double else slot == k
 
 
+def test_the_slots_of_the_dt_parameters():
+    """cfl, eta and kappa, which a step's list takes anew when they change."""
+    from wellbalanced_b200.engine import _DT_SLOTS
+
+    build.build()
+    types = _lib.SIGNATURES["wb_stable_dt"][:-1]
+    doubles = [k for k, t in enumerate(types) if t is _lib.c_double]
+    assert doubles[-3:] == list(range(_DT_SLOTS.start, _DT_SLOTS.stop))
+    assert len(doubles) == 7  # the mean field and gamma before them
+
+
 def test_wrong_names_and_counts_are_refused():
     build.build()
     with pytest.raises(_lib.WBError, match="no launch named"):

@@ -54,6 +54,10 @@ def _device_bytes(array, device, dtype):
     return torch.from_numpy(array.view(np.uint8).reshape(-1).copy()).to(device)
 
 
+#: the slots of cfl, eta and kappa among the arguments of `wb_stable_dt`
+_DT_SLOTS = slice(15, 18)
+
+
 class Engine:
     """Device pools + op lists of one hierarchy; the kernels' launch sequence."""
 
@@ -443,7 +447,9 @@ class Engine:
                         self.bad.zero_()
                     launches()
             return
-        key = (tuple(groups_potential), tuple(groups_all), dt_params, advance, clear_bad)
+        # the list holds the dt parameters in slots that are written when they change: one list
+        # for every cfl a run takes
+        key = (tuple(groups_potential), tuple(groups_all), dt_params is not None, advance, clear_bad)
         found = self._lists.get(key)
         if found is None:
             if self.max_level > 0 and self._uses_staged_fluxes():
@@ -455,12 +461,16 @@ class Engine:
                 if clear_bad:
                     self._launch("clear_bytes", self.bad.data_ptr(), 8)
                 launches()
-                found = (_lib.launch_list(self._recording), self.launches - before)
+                rows = [k for k, (name, *_) in enumerate(self._recording) if name == "wb_stable_dt"]
+                found = [_lib.launch_list(self._recording), self.launches - before, rows, dt_params]
             finally:
                 self._recording = None
                 self.launches = before
             self._lists[key] = found
-        entries, kernels = found
+        entries, kernels, rows, written = found
+        if written != dt_params:
+            entries["args"][rows, _DT_SLOTS] = np.array(dt_params, dtype=np.float64).view(np.int64)
+            found[3] = dt_params
         _lib.call("wb_run_launches", entries.ctypes.data, int(entries.size), int(count), self._s())
         self.launches += kernels * count
 
