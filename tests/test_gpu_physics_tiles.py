@@ -39,3 +39,28 @@ def test_terms_set_later_run_on_the_default_tiles(ndim, precision):
         stages.append(eng.stage_pool.clone())
     assert shapes[1] != shapes[0]  # the ideal model had chosen another shape
     assert torch.equal(*stages)
+
+
+@pytest.mark.parametrize("precision, sides", [(32, (32, 48, 64)), (64, (64, 80, (48, 33)))])
+def test_terms_set_on_a_batch_run_on_the_default_tiles(precision, sides):
+    from wellbalanced_b200 import Batch
+
+    stages, shapes = [], []
+    for tile in (None, "default"):
+        batch = Batch(sides, precision=precision)
+        shapes.append(tuple(batch.layout.tile_shape))
+        if tile == "default":
+            batch = Batch(sides, precision=precision, tile=batch.layout.default_tile)
+        for k, (nx, ny) in enumerate(batch.sides):
+            x, y = np.meshgrid((np.arange(nx) + 0.5) / nx, (np.arange(ny) + 0.5) / ny, indexing="ij")
+            xn, yn = np.meshgrid(np.arange(nx + 1) / nx, np.arange(ny + 1) / ny, indexing="ij")
+            rho = 1.0 + 0.1 * k + 0.2 * np.cos(2 * np.pi * x)
+            batch.set_instance(k, (rho, 0.3 * rho, -0.2 * rho * np.cos(2 * np.pi * y), 0.0 * rho, 2.0 + rho, 0.1 * rho),
+                               0.05 * np.sin(2 * np.pi * xn) * np.cos(2 * np.pi * yn))
+        batch.finish_state()
+        batch.engine.physics = (1e-3, 0.0, 0.0, 0.0, 0.0)
+        assert tuple(batch.layout.tile_shape) == tuple(batch.layout.default_tile)
+        batch.advance(2)
+        stages.append(batch.engine.state.clone())
+    assert shapes[0] != tuple(batch.layout.default_tile)  # the ideal batch had chosen another shape
+    assert torch.equal(*stages)

@@ -49,21 +49,23 @@ class Batch:
             self.hierarchies.append(h)
             layouts.append(layout)
         self.layout = Layout.merge(layouts)
+        if tile is None or tile == "auto":
+            self.layout.suit_tile()
         self.engine = Engine(None, precision=self.precision, limiter=LIMITER_CODES.index(limiter), gamma=self.gamma,
                              mean_field=(0.0, 0.0), device=device, layout=self.layout)
         self._patch_starts = np.cumsum([0] + [1] * self.count)
         self.steps = 0
         self._graph = None
-        # tile shape of the stage kernel: None (default), (tx, ty), or "auto" (tuned in
-        # finish_state, on the batch's own patch sizes)
+        # tile shape of the stage kernel: None (the one that suits the sides; non-ideal terms set
+        # on the engine take the default one), (tx, ty), or "auto" (tuned in finish_state, on the
+        # batch's own patch sizes)
         self._auto_tile = tile == "auto"
         self.tile = None if tile is None or self._auto_tile else tuple(tile)
         self.tile_timings = None
-        tile = self.layout.suited_tile() if self.tile is None else self.tile
-        if tile != self.layout.tile_shape:
+        if self.tile is not None and self.tile != self.layout.tile_shape:
             from wellbalanced_b200.autotune import _set_tile
 
-            _set_tile(self.engine, tile)
+            _set_tile(self.engine, self.tile)
 
     @classmethod
     def orszag_tang(cls, count, *, seed=0, precision=32, **options):

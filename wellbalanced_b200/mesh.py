@@ -568,6 +568,12 @@ class Layout:
         self.tile = self.tile_shape = tile
         self._cut_tiles()
 
+    def suit_tile(self):
+        """The 2D work list of a merged layout cut for the shape that suits its patches."""
+        self._suit_tile = True
+        if self.suited_tile() != self.tile_shape:
+            self._cut_tiles()
+
     def _cut_tiles(self):
         """The stage kernel's work list: every patch's computed cells and nodes in tiles (3D:
         columns of `march` cell planes)."""
