@@ -105,7 +105,15 @@ int wb_mhd_conductive(const double* prim, const double* bxf, const double* byf, 
 /*
  * dt: device double per instance. bad: device counter of bad cells (added to).
  * bflux: device double array of boundary-face fluxes (NULL to skip).
- * lx (3D only): cell planes per tile along x. */
+ * lx (3D only): cell planes per tile along x.
+ *
+ * Of PatchDesc.flags the stage kernels read bits 0 to 5 (walls: lower and upper face of axes
+ * 0, 1, 2), bits 8 to 10 (the patch computes its last node plane along that axis) and, in 2D,
+ * bit 11 (WRAP). WRAP is for a patch that is its own periodic neighbour along both axes: a lone
+ * patch that spans a fully periodic domain. dst then gets the patch's halo with its points, and
+ * no halo copies are needed before the next stage. The bit is ignored, and the copies are
+ * needed as for any other patch, where the patch has fewer than three cells along an axis or
+ * bit 8 or 9 is set. */
 int wb_stage2d(int precision, const void* src, const void* base, void* dst, const void* patches,
                const void* tiles, int ntiles, const double* dt, double gamma, double b0x, double b0y,
                int limiter, unsigned long long* bad, double* bflux, void* stream);

@@ -64,3 +64,26 @@ def test_a_batch_wraps_instance_by_instance():
     before = batch.engine.state.clone()
     batch.engine.fill(batch.engine.state)
     assert torch.equal(batch.engine.state, before)
+
+
+@pytest.mark.parametrize("precision", [32, 64, "mixed"])
+@pytest.mark.parametrize("shape, options", [((2, 8), {}), ((8, 2), {}), ((1, 5), {}), ((5, 1), {}),
+                                            ((16, 16), {"periodic": False})])
+def test_the_flag_is_ignored_where_an_image_has_no_single_writer(shape, options, precision):
+    """Fewer than three cells an axis, or a last node plane of the patch's own: the stage leaves
+    the halo to the fill, with the flag as without it."""
+    from wellbalanced_b200 import _lib
+    from wellbalanced_b200.engine import _device_bytes
+    from wellbalanced_b200.mesh import WRAP
+
+    eng = _model(shape, precision, **options).engine
+    eng.dt.fill_(1e-4)
+    pools = []
+    for flag in (0, WRAP):
+        rows = eng.layout.rows.copy()
+        rows["flags"] |= flag
+        eng.patches = _device_bytes(rows, eng.device, _lib.PATCH)
+        eng.stage_pool.fill_(7.0)
+        eng.stage(eng.state, None, eng.stage_pool)
+        pools.append(eng.stage_pool.clone())
+    assert torch.equal(*pools)

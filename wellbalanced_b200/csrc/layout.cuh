@@ -26,8 +26,9 @@ constexpr int kWallHi2 = 1 << 5;
 constexpr int kOwnLast0 = 1 << 8;  // the patch computes its last node plane along axis 0
 constexpr int kOwnLast1 = 1 << 9;
 constexpr int kOwnLast2 = 1 << 10;
-// the patch is its own periodic neighbour along every axis (it spans the domain; at least
-// three cells per axis): the 2D stage kernel writes each point's images into its halo as well
+// the patch is its own periodic neighbour along every axis (it spans the domain): the 2D stage
+// kernel writes each point's images into its halo as well, unless the patch has fewer than
+// three cells along an axis or owns a last node plane
 constexpr int kWrap = 1 << 11;
 // a dense block standing for a box of another rank's patch (mailboxes, proxies): the
 // copy, interpolation, restriction and face-flux kernels address it like the patch

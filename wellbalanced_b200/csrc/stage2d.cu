@@ -365,8 +365,10 @@ __global__ void __launch_bounds__(kThreads2D, (Occupancy2D<S, R>::kBlocks)) stag
   // pass of its own that tiles inside the patch skip: images written from the loop above,
   // with the values at hand, cost every tile (512 mixed planes: 803 -> 874 us a launch,
   // here 863 us, what the stage and the fill took apart). B200, stage + fill: 256^2 float64
-  // 19.9 -> 15.1 us, 501 x 339 float32 20.4 -> 16.8 us.
-  if (!(P.flags & kWrap) || (x0 >= 3 && x0 + TX <= nx - 2 && y0 >= 3 && y0 + TY <= ny - 2)) return;
+  // 19.9 -> 15.1 us, 501 x 339 float32 20.4 -> 16.8 us. The flag counts only where every image
+  // has one writer: three cells an axis, upper nodes that are images and not the patch's own.
+  const bool wraps = (P.flags & (kWrap | kOwnLast0 | kOwnLast1)) == kWrap && nx >= 3 && ny >= 3;
+  if (!wraps || (x0 >= 3 && x0 + TX <= nx - 2 && y0 >= 3 && y0 + TY <= ny - 2)) return;
 #pragma unroll 1
   for (int it = 0; it < NIT; ++it) {
     const int t = threadIdx.x + kThreads2D * it;
