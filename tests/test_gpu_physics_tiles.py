@@ -64,3 +64,24 @@ def test_terms_set_on_a_batch_run_on_the_default_tiles(precision, sides):
         stages.append(batch.engine.state.clone())
     assert shapes[0] != tuple(batch.layout.default_tile)  # the ideal batch had chosen another shape
     assert torch.equal(*stages)
+
+
+def test_a_captured_step_keeps_its_work_list():
+    """Terms set after a step was captured cut other tiles; the graph replays the ideal step with
+    the list it was captured with, whatever the allocator does with the memory of dropped ones."""
+    from wellbalanced_b200 import Batch
+
+    captured, ideal = Batch.orszag_tang(4, seed=3), Batch.orszag_tang(4, seed=3)
+    captured.capture()
+    tiles = captured.engine.tiles
+    assert captured._graph.tiles is tiles
+    captured.engine.physics = (1e-3, 0.0, 0.0, 0.0, 0.0)
+    assert captured.engine.tiles is not tiles
+    kept = tiles.data_ptr()
+    del tiles
+    others = [torch.zeros(captured.engine._ideal_tiles.numel(), dtype=torch.uint8, device="cuda") for _ in range(8)]
+    assert all(t.data_ptr() != kept for t in others)
+    captured.advance(2)
+    ideal.advance(3)
+    torch.cuda.synchronize()
+    assert torch.equal(captured.engine.state, ideal.engine.state)

@@ -198,6 +198,7 @@ class Engine:
             layout._suit_tile = False
             layout.tile_shape = layout.default_tile
             layout._cut_tiles()
+            self._ideal_tiles = self.tiles  # launches in flight on another stream may read it
             self.tiles = _device_bytes(layout.tiles, self.device, _lib.TILE)
             self.ntiles = int(layout.tiles.size)
 
@@ -418,6 +419,7 @@ class Engine:
         torch.cuda.current_stream(self.device).wait_stream(stream)
         torch.cuda.synchronize(self.device)
         graph = torch.cuda.CUDAGraph()
+        graph.tiles = self.tiles  # replayed with this work list, also where another replaces it
         with torch.cuda.graph(graph):
             step()
         torch.cuda.synchronize(self.device)
