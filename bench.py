@@ -64,9 +64,9 @@ def parse():
                              "halo exchange over NCCL, a global dt) instead of N replicas")
     parser.add_argument("--no-extra", action="store_true",
                         help="turbulence at one GPU: skip the batch and Harris configurations measured beside it")
-    parser.add_argument("--lx", default="auto", help="turbulence: x-planes per tile (an integer, or auto: tuned)")
+    parser.add_argument("--lx", default="auto", help="turbulence: x-planes per tile (an integer: at most that many; or auto: tuned)")
     parser.add_argument("--tile3d", default=None,
-                        help="turbulence with an integer --lx: the stage kernel's TYxTZ tile shape (default 16x16)")
+                        help="turbulence with an integer --lx: the stage kernel's TYxTZ tile shape (default: by the grid's size)")
     return parser.parse_args()
 
 
@@ -222,7 +222,6 @@ class Turbulence:
             from wellbalanced_b200.autotune import _set_tile
 
             _set_tile(self.engine, tuple(int(v) for v in args.tile3d.split("x")))
-        self.lx = self.model.lx
         self.cells = self.n**3
 
     #: the Mach-1 box leaves the method's positivity range after ~700 steps (in the
@@ -252,7 +251,7 @@ class Turbulence:
         return {
             "workload": self.describe(self.args),
             "cells_per_gpu": self.cells,
-            "tile": {"y": eng.layout.tile_shape[0], "z": eng.layout.tile_shape[1], "x_planes": self.lx},
+            "tile": {"y": eng.layout.tile_shape[0], "z": eng.layout.tile_shape[1], "x_planes": eng.layout.march},
             "autotune_ms_per_launch": describe(self.model.lx_timings),
         }
 
@@ -326,7 +325,6 @@ class PartitionedTurbulence(Turbulence):
         self.model._after_state()
         self.model._ready = True
         self.engine = self.model.engine
-        self.lx = lx
         self.cells = n**3
         self.model.lx_timings = None
 

@@ -77,7 +77,9 @@ class MHD3D:
         self.periodic = tuple(hierarchy.periodic)
         self.precision = _lib.precision_code(precision)
         self.device = device
-        # x-planes per tile of the stage kernel; "auto": tuned when the state is first set
+        # x-planes per tile of the stage kernel at most: a model of its cost takes fewer, and
+        # smaller tiles, where that many leave SMs idle (`march` is what runs); "auto": the tile
+        # and the planes tuned when the state is first set
         self._auto_lx = lx == "auto"
         self.lx = 32 if self._auto_lx else int(lx)
         self.lx_timings = None
@@ -96,6 +98,22 @@ class MHD3D:
     def _single_rank(self, what):
         if getattr(self, "_group", None) is not None:
             raise NotImplementedError(f"{what} on a hierarchy partitioned over ranks")
+
+    @property
+    def march(self) -> int:
+        """The x-planes per tile that the stage kernel runs with. Setting it takes exactly that
+        many, on the tiles as they are; a regrid chooses anew, at most `lx`."""
+        return self.engine.layout.march
+
+    @march.setter
+    def march(self, planes: int) -> None:
+        from wellbalanced_b200.autotune import _set_lx
+
+        if int(planes) < 1:
+            raise ValueError("a tile marches over at least one plane")
+        self._single_rank("march")
+        _set_lx(self.engine, planes)
+        self._graph = None
 
     #: whether steps run the fused stage kernel (False: the per-kernel float64 path)
     _fused = True
@@ -285,8 +303,9 @@ class MHD3D:
         self._after_state()
 
     def _after_state(self, tune=True):
-        """The halos and the restriction of a new state; with `tune`, the autotuner's x-plane
-        count (a regrid keeps the count tuned before it: `tune` False)."""
+        """The halos and the restriction of a new state; with `tune`, the autotuner's tile and
+        x-plane count (a regrid, `tune` False, cuts by the model, at most the count tuned before
+        it: the patches that count was timed on are gone)."""
         self.engine.dt_ready = False
         eng = self.engine
         if self.hierarchy.max_level > 0:
