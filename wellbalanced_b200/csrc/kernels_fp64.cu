@@ -25,7 +25,7 @@ __global__ void primitive_fp64_kernel(const double* __restrict__ rho, const doub
   const int i = int(t / (Y + 1));
   const int j = int(t % (Y + 1));
   const int A = Y + 1;  // row pitch of az
-  using M = Math<double>;
+  using M = MathIeee;
   const double idx = M::inv(dx), idy = M::inv(dy);
   if (j < Y) bxf[int64_t(i) * Y + j] = M::div(az[int64_t(i) * A + j + 1] - az[int64_t(i) * A + j], dy, idy) + b0x;
   if (i < X)
@@ -161,7 +161,7 @@ __global__ void rate_fp64_kernel(const double* __restrict__ rho, const double* _
     const int A = Y + 1;
     const int64_t c = int64_t(i) * Y + j;
     const double r = rho[c];
-    using M = Math<double>;
+    using M = MathIeee;
     const double ir = M::inv(r), idx = M::inv(dx), idy = M::inv(dy);
     const double u = M::div(mx[c], r, ir), v = M::div(my[c], r, ir), w = M::div(mz[c], r, ir);
     const double bx = 0.5 * (M::div(az[int64_t(i) * A + j + 1] - az[int64_t(i) * A + j], dy, idy) + b0x +
@@ -171,8 +171,8 @@ __global__ void rate_fp64_kernel(const double* __restrict__ rho, const double* _
     const double bzc = bz[c];
     const double p =
         (gamma - 1.0) * (energy[c] - 0.5 * r * (u * u + v * v + w * w) - 0.5 * (bx * bx + by * by + bzc * bzc));
-    rate = M::div(fabs(u) + fast_speed(r, p, bx, by, bzc, gamma), dx, idx) +
-           M::div(fabs(v) + fast_speed(r, p, by, bx, bzc, gamma), dy, idy);
+    rate = M::div(fabs(u) + fast_speed<double, M>(r, p, bx, by, bzc, gamma), dx, idx) +
+           M::div(fabs(v) + fast_speed<double, M>(r, p, by, bx, bzc, gamma), dy, idy);
     smallest = r;
   }
   block_reduce_keys(rate, smallest, keys);

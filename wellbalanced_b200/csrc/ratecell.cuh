@@ -53,8 +53,10 @@ struct RateMath<float> {
   static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
   static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
   static __device__ __forceinline__ float div(float a, float, float inv_b) { return __fmul_rn(a, inv_b); }
+  static __device__ __forceinline__ float quotient(float a, float b, float inv_b) { return div(a, b, inv_b); }
   // a / b + c and a / h - b / k
   static __device__ __forceinline__ float div_plus(float a, float, float inv_b, float c) { return __fmaf_rn(a, inv_b, c); }
+  static __device__ __forceinline__ float ratio_plus(float a, float b, float inv_b, float c) { return div_plus(a, b, inv_b, c); }
   static __device__ __forceinline__ float curl(float a, float, float ih, float b, float, float ik) {
     return __fmaf_rn(a, ih, -__fmul_rn(b, ik));
   }
@@ -69,8 +71,14 @@ struct RateMath<double> {
   static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
   static __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
   static __device__ __forceinline__ double div(double a, double b, double inv_b) { return Math<double>::div(a, b, inv_b); }
+  // a / b also where a is infinite: a signal speed without bound gives no step, not a NaN that
+  // the maximum passes over
+  static __device__ __forceinline__ double quotient(double a, double b, double inv_b) { return MathIeee::div(a, b, inv_b); }
   static __device__ __forceinline__ double div_plus(double a, double b, double inv_b, double c) {
     return __dadd_rn(div(a, b, inv_b), c);
+  }
+  static __device__ __forceinline__ double ratio_plus(double a, double b, double inv_b, double c) {
+    return __dadd_rn(quotient(a, b, inv_b), c);
   }
   static __device__ __forceinline__ double curl(double a, double h, double ih, double b, double k, double ik) {
     return __dadd_rn(div(a, h, ih), -div(b, k, ik));
@@ -131,10 +139,10 @@ __device__ __forceinline__ void rate_cells2d(const S* __restrict__ src, const Pa
     const S by = Q::mul(S(0.5), Q::add(Q::div_plus(a00 - a10, dx, idx, by0), Q::div_plus(a01 - a11, dx, idx, by0)));
     const S b2 = Q::fma(bz, bz, Q::fma(bx, bx, Q::mul(by, by)));
     const S p = rate_pressure(gm1, e, r, u, v, w, b2);
-    const S a2 = Q::div(Q::mul(g, p), r, ir);
+    const S a2 = Q::quotient(Q::mul(g, p), r, ir);
     const S cx = Q::add(rabs(u), rate_speed<S, 2>(a2, bx, b2, r, ir));
     const S cy = Q::add(rabs(v), rate_speed<S, 2>(a2, by, b2, r, ir));
-    largest = rmax(largest, Q::div_plus(cx, dx, idx, Q::div(cy, dy, idy)));
+    largest = rmax(largest, Q::ratio_plus(cx, dx, idx, Q::quotient(cy, dy, idy)));
     smallest = rmin(smallest, r);
   }
 }
@@ -177,11 +185,11 @@ __device__ __forceinline__ void rate_cells3d(const S* __restrict__ src, const Pa
     const S x2 = Q::mul(bx, bx), y2 = Q::mul(by, by), z2 = Q::mul(bz, bz);
     const S xy = Q::add(x2, y2), yz = Q::add(y2, z2), zx = Q::add(z2, x2);
     const S p = rate_pressure(gm1, src[4 * fs + o], r, u, v, w, Q::add(xy, z2));
-    const S a2 = Q::div(Q::mul(g, p), r, ir);
+    const S a2 = Q::quotient(Q::mul(g, p), r, ir);
     const S cx = Q::add(rabs(u), rate_speed<S, 3>(a2, bx, Q::add(xy, z2), r, ir));
     const S cy = Q::add(rabs(v), rate_speed<S, 3>(a2, by, Q::add(yz, x2), r, ir));
     const S cz = Q::add(rabs(w), rate_speed<S, 3>(a2, bz, Q::add(zx, y2), r, ir));
-    largest = rmax(largest, Q::div_plus(cz, dz, idz, Q::div_plus(cx, dx, idx, Q::div(cy, dy, idy))));
+    largest = rmax(largest, Q::ratio_plus(cz, dz, idz, Q::ratio_plus(cx, dx, idx, Q::quotient(cy, dy, idy))));
     smallest = rmin(smallest, r);
   }
 }
