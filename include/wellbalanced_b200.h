@@ -177,9 +177,9 @@ int wb_finalize_dt(const unsigned long long* keys, int ninstances, double cfl, d
                    double gamma, const double* inv_dx2_sum, double* time, const double* end, double* dt,
                    int advance, void* stream);
 
-/* wb_rate and wb_finalize_dt in one launch (with level_keys, inv_dx2_levels and nlevels:
- * wb_rate_levels and wb_finalize_dt_levels; level_keys NULL: without levels). The same keys,
- * level_keys and dt. scratch: 1 + 2 ninstances (+ ninstances nlevels) 64-bit words, a ticket
+/* wb_rate and wb_finalize_dt in one call, and in one launch up to 256 instances (with
+ * level_keys, inv_dx2_levels and nlevels: wb_rate_levels and wb_finalize_dt_levels; level_keys
+ * NULL: without levels). The same keys, level_keys and dt. scratch: 1 + 2 ninstances (+ ninstances nlevels) 64-bit words, a ticket
  * (0) and the identities of the keys (per instance 0x8000000000000000, 0xfff0000000000000;
  * per level 0xfff0000000000000); every launch leaves it so. Launches that share a scratch
  * must not overlap: of two that do (with the same work list) either may form its dt from a

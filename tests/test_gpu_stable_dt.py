@@ -99,3 +99,25 @@ def test_overlapping_launches_leave_the_scratch_whole():
     assert torch.equal(engine.dt_scratch, scratch)
     engine.stable_dt(0.4)
     assert torch.equal(engine.dt, expect)
+
+
+@pytest.mark.parametrize("count", [255, 256, 257, 513])
+@pytest.mark.parametrize("precision", [32, 64])
+def test_every_count_of_instances_has_the_same_dt(count, precision):
+    """One launch up to 256 instances, the rate and dt launches above."""
+    from wellbalanced_b200 import Batch
+    from wellbalanced_b200.problems import orszag_tang_2d
+
+    batch = Batch([(8, 20, 48)[k % 3] for k in range(count)], precision=precision)
+    for k, (n, _) in enumerate(batch.sides):
+        batch.set_instance(k, *orszag_tang_2d(n, 0.5 + k / count, 1.5 - k / count))
+    batch.finish_state()
+    engine = batch.engine
+    engine.rate()
+    engine.finalize_dt(0.4)
+    expect, keys = engine.dt.clone(), engine.keys.clone()
+    scratch = engine.dt_scratch.clone()
+    engine.dt.zero_()
+    engine.stable_dt(0.4)
+    assert torch.equal(engine.dt, expect) and torch.equal(engine.keys, keys)
+    assert torch.equal(engine.dt_scratch, scratch) and float(expect.min()) > 0.0

@@ -187,6 +187,13 @@ __global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4) stable_d
   }
 }
 
+// Instances up to which the last block makes every dt. More take the rate and dt launches: one
+// block walks them 256 at a time, and thousands of small blocks queue at the ticket. B200,
+// three launches and one, float32 (float64): 256 instances of 64^2 12.2 and 12.0 us (21.4 and
+// 22.4), 512 of 64^2 17.4 and 19.5 (40.6 and 43.1), 4096 of 16^2 17.4 and 29.7 (27.7 and 50.6),
+// 16384 of 16^2 57 and 124 (100 and 211).
+constexpr int kOneLaunchInstances = 256;
+
 // scratch: 1 + 2 ninstances (+ ninstances nlevels) words: the ticket (0), then (key(0),
 // key(+inf)) per instance and key(+inf) per level, as every launch leaves them.
 template <typename S>
@@ -195,6 +202,13 @@ int launch_stable_dt(const S* state, const PatchDesc* patches, int ndim, const i
                      int ninstances, unsigned long long* level_keys, int nlevels, double cfl, double eta, double kappa,
                      const double* inv_dx2_sum, const double* inv_dx2_levels, double* time, const double* end,
                      double* dt, int advance, unsigned long long* scratch, cudaStream_t stream) {
+  if (ninstances > kOneLaunchInstances) {
+    const int status = launch_rate_chunks<S>(state, patches, 0, ndim, chunk_patch, chunk_start, nchunks, b0, gamma, keys,
+                                             ninstances, stream, level_keys, nlevels);
+    return status != kOk ? status
+                         : launch_finalize_dt(keys, ninstances, cfl, eta, kappa, gamma, inv_dx2_sum, time, end, dt, advance,
+                                              stream, level_keys, inv_dx2_levels, nlevels);
+  }
   const RateSlots slots{scratch + 1, ninstances, level_keys ? scratch + 1 + 2 * ninstances : nullptr, nlevels, nullptr};
   const StableDt a{cfl, eta, kappa, gamma, inv_dx2_sum, inv_dx2_levels, time, end, dt, advance, keys, level_keys};
   unsigned* ticket = reinterpret_cast<unsigned*>(scratch);

@@ -8,7 +8,7 @@ through the C ABI:
   level: interpolation from the level below, same-level copies, outflow / wall faces;
 * ``restrict(pool, groups)`` — patchwork's ``restrict``;
 * ``stage(...)`` — one fused RK stage over every tile;
-* ``stable_dt()`` — the stable step on the device in one launch (``rate()`` and
+* ``stable_dt()`` — the stable step on the device in one call (``rate()`` and
   ``finalize_dt()`` apart where ranks reduce between them);
 * ``run_steps(...)`` — whole steps from a launch list put together once.
 
@@ -54,6 +54,8 @@ def _device_bytes(array, device, dtype):
     return torch.from_numpy(array.view(np.uint8).reshape(-1).copy()).to(device)
 
 
+#: instances up to which `wb_stable_dt` is one launch (kOneLaunchInstances of csrc/rate.cu)
+_ONE_LAUNCH_INSTANCES = 256
 #: the slots of cfl, eta and kappa among the arguments of `wb_stable_dt`
 _DT_SLOTS = slice(15, 18)
 
@@ -349,8 +351,9 @@ class Engine:
         self.launches += 1
 
     def stable_dt(self, cfl, eta=0.0, kappa=0.0, *, advance=False):
-        """`rate` of the state and `finalize_dt` in one launch (as for them, one stream at a time:
-        the keys and the dt are the engine's own)."""
+        """`rate` of the state and `finalize_dt` in one call, and in one launch up to
+        `_ONE_LAUNCH_INSTANCES` (as for them, one stream at a time: the keys and the dt are the
+        engine's own)."""
         b = self.mean_field
         levels = self.per_level_dt
         self._launch("wb_stable_dt", self.precision, self.ndim, self.state.data_ptr(), self.patches.data_ptr(),
@@ -359,7 +362,7 @@ class Engine:
                      self.nlevels if levels else 0, float(cfl), float(eta), float(kappa), self.inv_dx2_sum.data_ptr(),
                      self.inv_dx2_levels.data_ptr() if levels else None, self.time.data_ptr(), None, self.dt.data_ptr(),
                      int(advance), self.dt_scratch.data_ptr())
-        self.launches += 1
+        self.launches += 1 if self.ninstances <= _ONE_LAUNCH_INSTANCES else 3 if self.nchunks else 2
 
     def read_status(self):
         """(bad cells, times, dts) on the host, once the launches so far are done: one copy."""
