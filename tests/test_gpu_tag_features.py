@@ -57,3 +57,27 @@ def test_features_do_not_depend_on_the_blocks(shape, split, precision):
               tagger.mean.data_ptr(), tagger.inv_std.data_ptr(), flat.data_ptr() + 4,
               torch.cuda.current_stream().cuda_stream)
     assert torch.equal(flat[1:].reshape(rows.shape), rows)
+
+
+def test_a_ranks_rows_are_those_of_its_own_patches():
+    from types import SimpleNamespace
+
+    from wellbalanced_b200.distributed import LocalCluster
+    from wellbalanced_b200.tagger import LearnedTagger
+
+    whole = _model((16, 12, 20), (3, 2, 2), 64)
+    patches = whole.hierarchy.patches
+    tagger = LearnedTagger()
+    rows, starts = tagger.features(whole)
+    owner = [0, 1, 1, 0, 1, 0, 0, 1, 1, 1, 0, 1]
+    cluster = LocalCluster(whole.engine.layout, owner, precision=64, limiter=whole.engine.limiter)
+    for rank, engine in enumerate(cluster.engines):
+        mine = [k for k, r in enumerate(owner) if r == rank]
+        for local, k in enumerate(mine):
+            for f in range(8):
+                engine.view(engine.state, patches[k], f).copy_(whole.engine.view(whole.engine.state, patches[k], f))
+        got, first = tagger.features(SimpleNamespace(engine=engine, hierarchy=whole.hierarchy))
+        assert got.shape[0] == sum(int(np.prod(patches[k].shape)) for k in mine) and len(first) == len(mine)
+        for local, k in enumerate(mine):
+            n = int(np.prod(patches[k].shape))
+            assert torch.equal(got[int(first[local]) :][:n], rows[int(starts[k]) :][:n])

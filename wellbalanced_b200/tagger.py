@@ -66,11 +66,12 @@ class LearnedTagger:
         eng = model.engine
         if eng.ndim != 3:
             raise ValueError("the stencil features are defined on 3D hierarchies")
-        # the layout's patch table is in the hierarchy's patch order
-        ends = np.cumsum(np.prod(eng.layout.rows["n"][: len(model.hierarchy.patches)], axis=1, dtype=np.int64))
-        starts = np.concatenate([[0], ends[:-1]]).astype(np.int64)
+        # the layout's patch table is in the hierarchy's patch order (of a rank of a partition: its
+        # own patches, then the blocks that stand for other ranks')
+        ends = np.cumsum(np.prod(eng.layout.rows["n"][: eng.layout.npatches], axis=1, dtype=np.int64))
+        starts = np.concatenate([[0], ends])[:-1].astype(np.int64)
         row_start = torch.from_numpy(starts).to(self.device)
-        out = torch.empty((int(ends[-1]), FEATURES), dtype=torch.float32, device=self.device)
+        out = torch.empty((int(ends[-1]) if ends.size else 0, FEATURES), dtype=torch.float32, device=self.device)
         mean = torch.zeros_like(self.mean) if raw else self.mean
         inv_std = torch.ones_like(self.inv_std) if raw else self.inv_std
         b = eng.mean_field
