@@ -39,3 +39,15 @@ def test_an_overlapping_kernel_marks_tables_only_as_read_only(name):
     params, _ = _kernels()[name]
     marked = re.findall(r"const\s+(\w+)\s*\*\s*__restrict__\s*(\w+)", params)
     assert all(kind in TABLES for kind, _ in marked), marked
+
+
+@pytest.mark.parametrize("name", ["ops.cuh", "ratecell.cuh", "stage2d.cu", "stage3d.cu", "reflux.cu"])
+def test_helpers_of_these_kernels_mark_tables_only(name):
+    """The bodies that the kernels share with the op programs, whose phases write what later
+    ones read: no read-only pointer to a state or a dt there either."""
+    text = _sources()[name]
+    helpers = [params for _, params in re.findall(r"__device__ __forceinline__ \w+ (\w+)\(([^{;]*)\)\s*\{", text)]
+    assert helpers
+    marked = [m for params in helpers for m in re.findall(r"const\s+(\w+)\s*\*\s*__restrict__\s*(\w+)", params)]
+    assert all(kind in TABLES for kind, _ in marked), marked
+    assert not re.search(r"const\s+(?:S|R|double)\s*\*\s*__restrict__\s*\w+\s*=", text)

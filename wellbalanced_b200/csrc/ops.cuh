@@ -185,8 +185,8 @@ __device__ __forceinline__ void axis_weights(int node_axis, int g, int& c0, int&
 // NF cell-centred fields of one fine point: two coarse cells along every axis, all loads of
 // all fields before the stores; each field's terms in the order a0, a1, a2.
 template <typename S, int NDIM, int NF>
-__device__ __forceinline__ void interp_cells(S* __restrict__ pool, const S* __restrict__ coarse, int64_t cf, int64_t cp0,
-                                             int64_t cp1, const S (&w)[3][4], S* out, int64_t ff) {
+__device__ __forceinline__ void interp_cells(const S* coarse, int64_t cf, int64_t cp0, int64_t cp1,
+                                             const S (&w)[3][4], S* out, int64_t ff) {
   S acc[NF];
 #pragma unroll
   for (int f = 0; f < NF; ++f) acc[f] = S(0);
@@ -208,7 +208,7 @@ __device__ __forceinline__ void interp_cells(S* __restrict__ pool, const S* __re
 // One field of one fine point, any mix of node and cell axes (1, 2 or 4 coarse points along
 // an axis), terms in the order a0, a1, a2; the points of one a0 are loaded together.
 template <typename S, int NDIM>
-__device__ __forceinline__ S interp_value(const S* __restrict__ coarse, int64_t cp0, int64_t cp1, const int (&cnt)[3],
+__device__ __forceinline__ S interp_value(const S* coarse, int64_t cp0, int64_t cp1, const int (&cnt)[3],
                                           const S (&w)[3][4]) {
   constexpr int K2 = NDIM == 3 ? 4 : 1;
   S acc = S(0);
@@ -264,7 +264,7 @@ __device__ __forceinline__ void interp_points(S* __restrict__ pool, const PatchD
     const S* c = cbase + lo * cf + pitched(cp0, NDIM == 3 ? cp1 : 0, c0[0], c0[1], c0[2]);
     S* out = fbase + lo * ff + pitched(fp0, NDIM == 3 ? fp1 : 0, op.d[0] + q[0], op.d[1] + q[1], op.d[2] + q[2]);
     if (op.node_mask == 0 && nf == (NDIM == 3 ? 5 : 6)) {
-      interp_cells<S, NDIM, NDIM == 3 ? 5 : 6>(pool, c, cf, cp0, cp1, w, out, ff);
+      interp_cells<S, NDIM, NDIM == 3 ? 5 : 6>(c, cf, cp0, cp1, w, out, ff);
     } else {
 #pragma unroll 1
       for (int f = 0; f < nf; ++f) out[f * ff] = interp_value<S, NDIM>(c + f * cf, cp0, cp1, cnt, w);
@@ -335,7 +335,7 @@ __device__ __forceinline__ void restrict_op(S* __restrict__ pool, const PatchDes
 template <typename S, int NT>
 __device__ __forceinline__ void reflux_op(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
                                           const RefluxOp& op, double* __restrict__ reg,
-                                          const double* __restrict__ dt) {
+                                          const double* dt) {
   const PatchDesc C = patches[op.coarse];
   const double scale = 0.5 * dt[C.instance];
   const int64_t count = int64_t(op.len) * op.ncomp;

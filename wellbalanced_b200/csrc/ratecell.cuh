@@ -111,7 +111,7 @@ __device__ __forceinline__ S rate_pressure(S gm1, S e, S rho, S u, S v, S w, S f
 // a float32 3D cell against 32 bytes); unrolling by two raises the registers and loses warps.
 // 2D:
 template <typename S, int NT>
-__device__ __forceinline__ void rate_cells2d(const S* __restrict__ src, const PatchDesc& P, unsigned begin, int rounds,
+__device__ __forceinline__ void rate_cells2d(const S* src, const PatchDesc& P, unsigned begin, int rounds,
                                              double b0x, double b0y, double gamma, S& largest, S& smallest) {
   const int64_t pitch = P.pitch0, fs = P.fstride;
   using M = Math<S>;
@@ -149,7 +149,7 @@ __device__ __forceinline__ void rate_cells2d(const S* __restrict__ src, const Pa
 
 // 3D:
 template <typename S, int NT>
-__device__ __forceinline__ void rate_cells3d(const S* __restrict__ src, const PatchDesc& P, unsigned begin, int rounds,
+__device__ __forceinline__ void rate_cells3d(const S* src, const PatchDesc& P, unsigned begin, int rounds,
                                              double b0x, double b0y, double b0z, double gamma, S& largest, S& smallest) {
   const int64_t p0 = P.pitch0, p1 = P.pitch1, fs = P.fstride;
   using M = Math<S>;
@@ -199,7 +199,7 @@ __device__ __forceinline__ void rate_cells3d(const S* __restrict__ src, const Pa
 // (exact: the max of the float rates converts to the max of their double images), converted
 // once for the block reduction. 2D:
 template <typename S, int NT>
-__device__ __forceinline__ void rate_chunk2d(const S* __restrict__ pool, const PatchDesc* patches, int pi,
+__device__ __forceinline__ void rate_chunk2d(const S* pool, const PatchDesc* patches, int pi,
                                              int chunk_start, double b0x, double b0y, double gamma,
                                              const RateSlots& slots) {
   const PatchDesc P = patches[pi];
@@ -212,7 +212,7 @@ __device__ __forceinline__ void rate_chunk2d(const S* __restrict__ pool, const P
 
 // 3D:
 template <typename S, int NT>
-__device__ __forceinline__ void rate_chunk3d(const S* __restrict__ pool, const PatchDesc* patches, int pi,
+__device__ __forceinline__ void rate_chunk3d(const S* pool, const PatchDesc* patches, int pi,
                                              int chunk_start, double b0x, double b0y, double b0z, double gamma,
                                              const RateSlots& slots) {
   const PatchDesc P = patches[pi];
