@@ -38,9 +38,8 @@ template <typename S>
 constexpr int kInterpBlocks = sizeof(S) == 4 ? 16 : 12;
 
 template <typename S>
-__global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>) interp_ops_kernel(S* __restrict__ pool,
-                                                               const PatchDesc* __restrict__ patches,
-                                                               const InterpOp* __restrict__ ops) {
+__global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>)
+    interp_ops_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches, const InterpOp* __restrict__ ops) {
   after_previous();
   interp_op(pool, patches, ops[blockIdx.x]);
 }
@@ -50,9 +49,9 @@ __global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>) interp_ops_kerne
 // that another op of the launch writes or reads, as for interpolation ops trimmed to the
 // halo points no sibling covers (the copies read only their sources' computed points).
 template <typename S>
-__global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>) fill_ops_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches,
-                                                             const InterpOp* __restrict__ interp, int ninterp,
-                                                             const CopyOp* __restrict__ copies) {
+__global__ void __launch_bounds__(kOpThreads, kInterpBlocks<S>)
+    fill_ops_kernel(S* __restrict__ pool, const PatchDesc* __restrict__ patches, const InterpOp* __restrict__ interp,
+                    int ninterp, const CopyOp* __restrict__ copies) {
   after_previous();
   if (int(blockIdx.x) < ninterp)
     interp_op(pool, patches, interp[blockIdx.x]);

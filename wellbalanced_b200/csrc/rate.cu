@@ -118,11 +118,10 @@ struct StableDt {
 
 // (float32: 32 registers, 64 warps an SM, as the rate kernel alone)
 template <typename S, int NDIM>
-__global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4) stable_dt_kernel(const S* pool, const PatchDesc* patches,
-                                                                 const int* chunk_patch, const int* chunk_start,
-                                                                 int nchunks, int parts, double b0x, double b0y,
-                                                                 double b0z, const RateSlots scratch,
-                                                                 unsigned* ticket, const StableDt a) {
+__global__ void __launch_bounds__(kRateThreads, sizeof(S) == 4 ? 8 : 4)
+    stable_dt_kernel(const S* pool, const PatchDesc* patches, const int* chunk_patch, const int* chunk_start,
+                     int nchunks, int parts, double b0x, double b0y, double b0z, const RateSlots scratch,
+                     unsigned* ticket, const StableDt a) {
   after_previous();
   __shared__ double s_largest[kRateThreads / 32], s_smallest[kRateThreads / 32];
   __shared__ bool s_last;
@@ -218,11 +217,11 @@ int launch_stable_dt(const S* state, const PatchDesc* patches, int ndim, const i
   while (parts > 1 && int64_t(nchunks) * parts > 148 * 4) parts /= 2;
   const int grid = max(nchunks * parts, 1);
   if (ndim == 2)
-    launch_after(stable_dt_kernel<S, 2>, grid, kRateThreads, 0, stream, state, patches, chunk_patch, chunk_start, nchunks, parts,
-                                                             b0[0], b0[1], b0[2], slots, ticket, a);
+    launch_after(stable_dt_kernel<S, 2>, grid, kRateThreads, 0, stream, state, patches, chunk_patch, chunk_start,
+                 nchunks, parts, b0[0], b0[1], b0[2], slots, ticket, a);
   else
-    launch_after(stable_dt_kernel<S, 3>, grid, kRateThreads, 0, stream, state, patches, chunk_patch, chunk_start, nchunks, parts,
-                                                             b0[0], b0[1], b0[2], slots, ticket, a);
+    launch_after(stable_dt_kernel<S, 3>, grid, kRateThreads, 0, stream, state, patches, chunk_patch, chunk_start,
+                 nchunks, parts, b0[0], b0[1], b0[2], slots, ticket, a);
   return check_launch("stable_dt");
 }
 

@@ -276,11 +276,10 @@ constexpr int kFluxWarps = kFluxThreads / 32;
 inline int flux_splits(int nops) { return max(1, min(32, 148 * 64 / max(nops, 1))); }
 
 template <typename S, typename R, int LIM, bool PHYS>
-__global__ void __launch_bounds__(kFluxThreads) face_flux_ops_kernel(const S* pool,
-                                                                     const PatchDesc* __restrict__ patches,
-                                                                     const FaceFluxOp* __restrict__ ops, int nops,
-                                                                     int splits, double b0x, double b0y, double b0z, double gamma,
-                                                                     FacePhysics phys, double* __restrict__ reg) {
+__global__ void __launch_bounds__(kFluxThreads)
+    face_flux_ops_kernel(const S* pool, const PatchDesc* __restrict__ patches, const FaceFluxOp* __restrict__ ops,
+                         int nops, int splits, double b0x, double b0y, double b0z, double gamma, FacePhysics phys,
+                         double* __restrict__ reg) {
   after_previous();
   __shared__ double g_all[kFluxWarps][32][6];
   const int warp = threadIdx.x / 32, t = threadIdx.x % 32;
@@ -389,10 +388,22 @@ void launch_face_flux_staged(const S* pool, const PatchDesc* patches, const Face
   if (nfaces <= 0) return;
   const int grid = (nfaces + kStagedThreads - 1) / kStagedThreads;
   switch (limiter) {
-    case 0: launch_after(face_flux_staged_kernel<S, R, 0>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
-    case 1: launch_after(face_flux_staged_kernel<S, R, 1>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
-    case 2: launch_after(face_flux_staged_kernel<S, R, 2>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
-    default: launch_after(face_flux_staged_kernel<S, R, 3>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops, nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg); break;
+    case 0:
+      launch_after(face_flux_staged_kernel<S, R, 0>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops,
+                   nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg);
+      break;
+    case 1:
+      launch_after(face_flux_staged_kernel<S, R, 1>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops,
+                   nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg);
+      break;
+    case 2:
+      launch_after(face_flux_staged_kernel<S, R, 2>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops,
+                   nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg);
+      break;
+    default:
+      launch_after(face_flux_staged_kernel<S, R, 3>, grid, kStagedThreads, 0, stream, pool, patches, ops, nops,
+                   nfaces, b0[0], b0[1], b0[2], gamma, bflux, reg);
+      break;
   }
 }
 
@@ -403,10 +414,22 @@ void launch_face_flux_kernel(const S* pool, const PatchDesc* patches, const Face
   const int splits = flux_splits(nops);
   const int grid = int((int64_t(nops) * splits + kFluxWarps - 1) / kFluxWarps);
   switch (limiter) {
-    case 0: launch_after(face_flux_ops_kernel<S, R, 0, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    case 1: launch_after(face_flux_ops_kernel<S, R, 1, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    case 2: launch_after(face_flux_ops_kernel<S, R, 2, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
-    default: launch_after(face_flux_ops_kernel<S, R, 3, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops, splits, b0[0], b0[1], b0[2], gamma, phys, reg); break;
+    case 0:
+      launch_after(face_flux_ops_kernel<S, R, 0, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops,
+                   splits, b0[0], b0[1], b0[2], gamma, phys, reg);
+      break;
+    case 1:
+      launch_after(face_flux_ops_kernel<S, R, 1, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops,
+                   splits, b0[0], b0[1], b0[2], gamma, phys, reg);
+      break;
+    case 2:
+      launch_after(face_flux_ops_kernel<S, R, 2, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops,
+                   splits, b0[0], b0[1], b0[2], gamma, phys, reg);
+      break;
+    default:
+      launch_after(face_flux_ops_kernel<S, R, 3, PHYS>, grid, kFluxThreads, 0, stream, pool, patches, ops, nops,
+                   splits, b0[0], b0[1], b0[2], gamma, phys, reg);
+      break;
   }
 }
 

@@ -39,7 +39,8 @@ inline int check_launch(const char* what) {
 // read-only path, or before the call, and the kernel before may still be writing it. So such
 // a parameter is for tables that no launch writes (patches, op lists); the pools, the dt, the
 // flux register and the boundary fluxes are not marked so. B200: the refined sheet (25 launches a step)
-// 542 -> 476 us for two steps, 256^2 float64 (3 a step) 214 -> 200 us for four.
+// 542 -> 476 us for two steps, 256^2 float64 (3 a step) 214 -> 200 us for four. A launch that is
+// refused leaves its error for the `check_launch` after it.
 template <typename... P, typename... A>
 inline void launch_after(void (*kernel)(P...), int64_t grid, int threads, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t config = {};
