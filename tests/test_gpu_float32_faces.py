@@ -47,6 +47,37 @@ def test_a_flow_without_pressure_stays_finite(ndim, axis):
     assert torch.equal(model.engine.state, before)
 
 
+@pytest.mark.parametrize("ndim, axis", [(2, 0), (2, 1), (3, 0), (3, 1), (3, 2)])
+def test_a_negative_pressure_beside_a_cold_flow_keeps_the_upwind_flux(ndim, axis):
+    """Two cold supersonic streams, the faster one with a (bad) negative pressure: where they part
+    its star denominator is zero in float32, and the flux is that of the slower stream, as in
+    float64. Bound: float32 rounding of a flux (1e-6 of its scale) on the two faces of a cell."""
+    from wellbalanced_b200 import MHD2D, MHD3D
+    from wellbalanced_b200.mesh import AMRHierarchy
+
+    shape, ratio = (24, 24, 24)[:ndim], 0.02
+    fast = np.broadcast_to(np.moveaxis((np.arange(24) >= 12).reshape(24, *(1,) * (ndim - 1)), 0, axis), shape)
+    v = [np.full(shape, 0.5), np.full(shape, 0.25), np.full(shape, -0.75)]
+    v[axis] = np.where(fast, 6.0, 2.0)
+    cells = [np.ones(shape), *v, 1.5 * np.where(fast, -2e-14, 4e-15) + 0.5 * sum(c * c for c in v)]
+    results = []
+    for precision in (64, "mixed"):
+        mesh = AMRHierarchy(shape, periodic=(True,) * ndim)
+        model = (MHD2D if ndim == 2 else MHD3D)(mesh, precision=precision, limiter="minmod")
+        if ndim == 2:
+            model.set_conserved([*cells, np.zeros(shape)], np.zeros((25, 25)))
+        else:
+            model.set_conserved(cells, [np.zeros(tuple(24 + (a != c) for a in range(3))) for c in range(3)])
+        eng = model.engine
+        eng.dt.fill_(ratio / 24)
+        eng.stage(eng.state, None, eng.stage_pool)
+        results.append([model._read(mesh.patches[0], f, pool=eng.stage_pool).cpu().numpy() for f in range(5)])
+    scale = float(np.abs(cells[4]).max()) * 6.0
+    for want, got in zip(*results, strict=True):
+        assert np.isfinite(got).all()
+        assert np.abs(got - want).max() <= 2 * ratio * 1e-6 * scale
+
+
 @pytest.mark.parametrize("limiter", ["minmod", "vanleer", "mc"])
 @pytest.mark.parametrize("speed", [0.3, 4.0])
 @pytest.mark.parametrize("field", ["none", "normal", "across", "out"])

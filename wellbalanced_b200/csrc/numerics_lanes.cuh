@@ -147,9 +147,10 @@ __device__ __forceinline__ void hlld_front_lr(const float (&L)[7], const float (
   o.btl1 = bt1.v.x, o.btr1 = bt1.v.y;
   o.btl2 = bt2.v.x, o.btr2 = bt2.v.y;
   o.inv_sl = inv_ssm.v.x, o.inv_sr = inv_ssm.v.y;
-  // (written so that a NaN, a zero denominator and a side without a star state are redone too)
+  // (written so that a NaN, a zero denominator, also under a negative pressure, and a side without
+  // a star state are redone too)
   const float extent = fabsf(inv_ssm.v.x) + fabsf(inv_ssm.v.y) + fabsf(o.sm.v);
-  if (!any(!(labs(den) > F2(kNearDegenerate32) * (pt2 + F2(bn2.v)))) && extent < INFINITY) return;
+  if (!any(!(labs(den) > labs(F2(kNearDegenerate32) * (pt2 + F2(bn2.v))))) && extent < INFINITY) return;
   double Ld[7], Rd[7];
 #pragma unroll
   for (int c = 0; c < 7; ++c) {
