@@ -81,10 +81,12 @@ def test_a_negative_pressure_beside_a_cold_flow_keeps_the_upwind_flux(ndim, axis
 @pytest.mark.parametrize("limiter", ["minmod", "vanleer", "mc"])
 @pytest.mark.parametrize("speed", [0.3, 4.0])
 @pytest.mark.parametrize("field", ["none", "normal", "across", "out"])
-def test_faces_agree_with_float64(field, speed, limiter):
+@pytest.mark.parametrize("unit", [1.0, 2.0**-33])
+def test_faces_agree_with_float64(unit, field, speed, limiter):
     """Random cells with constant stripes (slopes of both signs, and zero) under a field that is
     absent, along x (B_n = 0 on the y-faces, a vanishing star denominator on the x-faces, whose
-    fast speed is the Alfven speed), along y, or along z (B_n = 0 everywhere).
+    fast speed is the Alfven speed), along y, or along z (B_n = 0 everywhere); and the same in units
+    in which the speeds are 1e-10 (their fourth powers are subnormal, good to 1e-6).
 
     Bound: a float32 flux is good to 2e-3 of its scale (star denominators are used down to 1e-3
     of their terms, with 1e-6 of rounding in them), four faces change a cell by dt / dx = 0.02 of
@@ -97,10 +99,11 @@ def test_faces_agree_with_float64(field, speed, limiter):
     rng = np.random.default_rng(5)
     stripes = (np.arange(shape[0]) // 4 % 3 == 0)[:, None]
     draw = lambda lo, hi: np.where(stripes, 0.5 * (lo + hi), rng.uniform(lo, hi, shape))  # noqa: E731
-    rho, p = draw(0.6, 1.4), draw(0.6, 1.4)
-    velocity = [draw(-speed, speed) for _ in range(3)]
+    rho, p = draw(0.6, 1.4), draw(0.6, 1.4) * unit**2
+    velocity = [draw(-speed, speed) * unit for _ in range(3)]
     mean, bz = {"none": ((0.0, 0.0), 0.0), "normal": ((2.0, 0.0), 0.0), "across": ((0.0, -2.0), 0.0),
                 "out": ((0.0, 0.0), 1.5)}[field]
+    mean, bz = (mean[0] * unit, mean[1] * unit), bz * unit
     b2 = mean[0] ** 2 + mean[1] ** 2 + bz**2
     energy = 1.5 * p + 0.5 * rho * sum(v * v for v in velocity) + 0.5 * b2
     results = []
@@ -109,14 +112,15 @@ def test_faces_agree_with_float64(field, speed, limiter):
         model = MHD2D(mesh, precision=precision, limiter=limiter, mean_field=mean)
         model.set_conserved([rho, *(rho * v for v in velocity), energy, np.full(shape, bz)], np.zeros((25, 41)))
         eng = model.engine
-        eng.dt.fill_(ratio * 0.025)
+        eng.dt.fill_(ratio * 0.025 / unit)
         eng.bad.zero_()
         eng.stage(eng.state, None, eng.stage_pool)
         assert int(eng.bad.item()) == 0
         (patch,) = mesh.patches
         results.append([model._read(patch, f, node=f == 6, pool=eng.stage_pool).cpu().numpy() for f in range(7)])
-    signal = speed + np.sqrt((5.0 / 3.0 * 1.4 + b2) / 0.6)
-    bound = 4 * ratio * 2e-3 * float(np.abs(energy).max()) * signal
-    for want, got in zip(*results, strict=True):
+    signal = speed + np.sqrt((5.0 / 3.0 * 1.4 + b2 / unit**2) / 0.6)
+    bound = 4 * ratio * 2e-3 * float(np.abs(energy).max()) / unit**2 * signal
+    scales = (1.0, unit, unit, unit, unit**2, unit, unit)
+    for want, got, scale in zip(*results, scales, strict=True):
         assert np.isfinite(got).all()
-        assert np.abs(got - want).max() <= bound
+        assert np.abs(got - want).max() <= bound * scale

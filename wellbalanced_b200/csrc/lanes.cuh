@@ -54,6 +54,7 @@ __device__ __forceinline__ L1 lcopysign(L1 m, L1 s) { return L1(copysignf(m.v, s
 // reciprocal and reciprocal square root from the special-function unit (~1 ulp)
 __device__ __forceinline__ L1 linv(L1 a) { return L1(rcp_ftz(a.v)); }
 __device__ __forceinline__ L1 lrsqrt(L1 a) { return L1(rsqrt_ftz(a.v)); }
+__device__ __forceinline__ L1 lrsqrt_subnormal(L1 a) { return L1(rsqrtf(a.v)); }
 __device__ __forceinline__ bool any(bool m) { return m; }
 
 struct M2 {
@@ -108,6 +109,7 @@ __device__ __forceinline__ F2 lmax3(F2 a, F2 b, F2 c) {
 __device__ __forceinline__ F2 lcopysign(F2 m, F2 s) { return F2(copysignf(m.v.x, s.v.x), copysignf(m.v.y, s.v.y)); }
 __device__ __forceinline__ F2 linv(F2 a) { return F2(rcp_ftz(a.v.x), rcp_ftz(a.v.y)); }
 __device__ __forceinline__ F2 lrsqrt(F2 a) { return F2(rsqrt_ftz(a.v.x), rsqrt_ftz(a.v.y)); }
+__device__ __forceinline__ F2 lrsqrt_subnormal(F2 a) { return F2(rsqrtf(a.v.x), rsqrtf(a.v.y)); }
 // a b rounded on its own also where a sum follows: ptxas fuses a packed product into a packed
 // sum (the scalar intrinsics it leaves alone)
 __device__ __forceinline__ L1 lproduct(L1 a, L1 b) { return a * b; }

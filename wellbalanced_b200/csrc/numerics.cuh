@@ -33,7 +33,7 @@ __device__ __forceinline__ double rcopysign(double m, double s) { return copysig
 // Reciprocal and reciprocal square root from the special-function unit (~1 ulp), flushing
 // subnormal operands: __fdividef and rsqrtf handle those with three to four more
 // instructions each, ~50 of a float32 face's ~600. An operand below 1.2e-38 gives infinity
-// here; square roots take it as zero.
+// here; roots of fourth powers of speeds, which reach that, take rsqrtf.
 __device__ __forceinline__ float rcp_ftz(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -92,7 +92,7 @@ template <>
 struct Math<float> {
   static __device__ __forceinline__ float inv(float b) { return rcp_ftz(b); }
   static __device__ __forceinline__ float div(float a, float, float inv_b) { return a * inv_b; }
-  static __device__ __forceinline__ float sqrt(float x) { return x >= kSmallestNormal ? x * rsqrt_ftz(x) : 0.0f; }
+  static __device__ __forceinline__ float sqrt(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
   static __device__ __forceinline__ float over_sqrt(float a, float sq) { return a * rcp_ftz(sq); }
 };
 

@@ -23,12 +23,20 @@ namespace wb {
 // the 256^3 box 1.98 ms with those, 1.74 now; of 512 2D instances of 32^2 to 256^2 cells, 0.90
 // and 0.81 ms.
 
-// sqrt(x) as x rsqrt(x); x below the smallest normal (zero and negative discriminants) counts
-// as that, so the root of zero is 1e-19: far under the rounding of what it is added to.
+// sqrt(x) as x rsqrt(x) of a density or a squared speed; x below the smallest normal counts as
+// that, so the root of zero is 1e-19.
 template <typename V>
 __device__ __forceinline__ V lsqrt(V x) {
   const V y = lmax(x, V(kSmallestNormal));
   return lproduct(y, lrsqrt(y));
+}
+
+// The same over all of float32, zero for zero and below: of fourth powers of speeds, which are
+// subnormal for speeds of 3e-10 in the user's units.
+template <typename V>
+__device__ __forceinline__ V lsqrt_subnormal(V x) {
+  const V y = lmax(x, V(0.0f));
+  return lproduct(y, lmin(lrsqrt_subnormal(y), V(3.0e38f)));
 }
 
 // Half the limited slope of a cell from its backward (a) and forward (b) differences. minmod
@@ -55,7 +63,7 @@ __device__ __forceinline__ V fast_speed_l(V rho, V p, V bn, V bt1, V bt2, V gamm
   const V b2 = fma(bt1, bt1, fma(bt2, bt2, bn2)) * ir;
   const V s = a2 + b2;
   const V disc = fma(V(-4.0f) * a2 * ir, bn2, s * s);
-  return lsqrt(V(0.5f) * (s + lsqrt(disc)));
+  return lsqrt(V(0.5f) * (s + lsqrt_subnormal(disc)));
 }
 
 // Conserved state and normal flux of a normal-frame primitive state; returns p_T.

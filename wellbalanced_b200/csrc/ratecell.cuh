@@ -61,7 +61,7 @@ struct RateMath<float> {
     return __fmaf_rn(a, ih, -__fmul_rn(b, ik));
   }
   static __device__ __forceinline__ float sqrt(float x) {
-    return x >= kSmallestNormal ? __fmul_rn(x, rsqrt_ftz(x)) : 0.0f;
+    return x > 0.0f ? __fmul_rn(x, rsqrtf(x)) : 0.0f;
   }
 };
 
