@@ -48,13 +48,18 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
+// the larger, or NaN where one is
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
 __device__ __forceinline__ L1 lmin3(L1 a, L1 b, L1 c) { return L1(min3(a.v, b.v, c.v)); }
 __device__ __forceinline__ L1 lmax3(L1 a, L1 b, L1 c) { return L1(max3(a.v, b.v, c.v)); }
 __device__ __forceinline__ L1 lcopysign(L1 m, L1 s) { return L1(copysignf(m.v, s.v)); }
 // reciprocal and reciprocal square root from the special-function unit (~1 ulp)
 __device__ __forceinline__ L1 linv(L1 a) { return L1(rcp_ftz(a.v)); }
 __device__ __forceinline__ L1 lrsqrt(L1 a) { return L1(rsqrt_ftz(a.v)); }
-__device__ __forceinline__ L1 lrsqrt_subnormal(L1 a) { return L1(rsqrtf(a.v)); }
 __device__ __forceinline__ bool any(bool m) { return m; }
 
 struct M2 {
@@ -109,7 +114,6 @@ __device__ __forceinline__ F2 lmax3(F2 a, F2 b, F2 c) {
 __device__ __forceinline__ F2 lcopysign(F2 m, F2 s) { return F2(copysignf(m.v.x, s.v.x), copysignf(m.v.y, s.v.y)); }
 __device__ __forceinline__ F2 linv(F2 a) { return F2(rcp_ftz(a.v.x), rcp_ftz(a.v.y)); }
 __device__ __forceinline__ F2 lrsqrt(F2 a) { return F2(rsqrt_ftz(a.v.x), rsqrt_ftz(a.v.y)); }
-__device__ __forceinline__ F2 lrsqrt_subnormal(F2 a) { return F2(rsqrtf(a.v.x), rsqrtf(a.v.y)); }
 // a b rounded on its own also where a sum follows: ptxas fuses a packed product into a packed
 // sum (the scalar intrinsics it leaves alone)
 __device__ __forceinline__ L1 lproduct(L1 a, L1 b) { return a * b; }

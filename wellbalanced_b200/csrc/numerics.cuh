@@ -33,7 +33,7 @@ __device__ __forceinline__ double rcopysign(double m, double s) { return copysig
 // Reciprocal and reciprocal square root from the special-function unit (~1 ulp), flushing
 // subnormal operands: __fdividef and rsqrtf handle those with three to four more
 // instructions each, ~50 of a float32 face's ~600. An operand below 1.2e-38 gives infinity
-// here; roots of fourth powers of speeds, which reach that, take rsqrtf.
+// here; the rate's roots of fourth powers of speeds, which reach that, take rsqrtf.
 __device__ __forceinline__ float rcp_ftz(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -108,7 +108,9 @@ struct MathRefined {
   static __device__ __forceinline__ double div(double a, double, double inv_b) { return a * inv_b; }
   static __device__ __forceinline__ double sqrt(double x) {
     if (!(x > 0.0)) return 0.0;
-    const double r0 = double(rsqrtf(float(x)));
+    const float f = float(x);
+    double r0 = double(rsqrtf(f));
+    if (f < 1.0e-30f) r0 = double(rsqrtf(float(x * 0x1p120))) * 0x1p60;  // fourth powers of small speeds
     return x * (r0 * (1.5 - 0.5 * x * r0 * r0));
   }
   static __device__ __forceinline__ double over_sqrt(double a, double sq) { return a * inv(sq); }

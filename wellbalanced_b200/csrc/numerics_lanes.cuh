@@ -23,20 +23,12 @@ namespace wb {
 // the 256^3 box 1.98 ms with those, 1.74 now; of 512 2D instances of 32^2 to 256^2 cells, 0.90
 // and 0.81 ms.
 
-// sqrt(x) as x rsqrt(x) of a density or a squared speed; x below the smallest normal counts as
-// that, so the root of zero is 1e-19.
+// sqrt(x) of a density as x rsqrt(x); x below the smallest normal counts as that, so the root of
+// zero is 1e-19.
 template <typename V>
 __device__ __forceinline__ V lsqrt(V x) {
   const V y = lmax(x, V(kSmallestNormal));
   return lproduct(y, lrsqrt(y));
-}
-
-// The same over all of float32, zero for zero and below: of fourth powers of speeds, which are
-// subnormal for speeds of 3e-10 in the user's units.
-template <typename V>
-__device__ __forceinline__ V lsqrt_subnormal(V x) {
-  const V y = lmax(x, V(0.0f));
-  return lproduct(y, lmin(lrsqrt_subnormal(y), V(3.0e38f)));
 }
 
 // Half the limited slope of a cell from its backward (a) and forward (b) differences. minmod
@@ -54,7 +46,11 @@ __device__ __forceinline__ V half_slope_l(V a, V b) {
   return lmax(lmin3(a, b, quarter), V(0.0f)) + lmin(lmax3(a, b, quarter), V(0.0f));
 }
 
-// Fast magnetosonic speed along the normal (the discriminant clipped at zero).
+// Fast magnetosonic speed along the normal. The two roots are x rsqrt(x) as it comes: NaN where x
+// is zero, negative or below the smallest normal (the discriminant, a fourth power of a speed, is
+// that at speeds of 3e-10 in the user's units), and such a face is redone in float64. B200, a step,
+// roots floored / by rsqrtf over all of float32 / as here: 256^3 3.98, 4.02 and 3.97 ms, 150 x 97 x
+// 75 mixed 1.039, 1.045 and 1.025 ms; 512 planes, two steps 3.75, 3.77 and 3.76 ms.
 template <typename V>
 __device__ __forceinline__ V fast_speed_l(V rho, V p, V bn, V bt1, V bt2, V gamma) {
   const V ir = linv(rho);
@@ -63,7 +59,8 @@ __device__ __forceinline__ V fast_speed_l(V rho, V p, V bn, V bt1, V bt2, V gamm
   const V b2 = fma(bt1, bt1, fma(bt2, bt2, bn2)) * ir;
   const V s = a2 + b2;
   const V disc = fma(V(-4.0f) * a2 * ir, bn2, s * s);
-  return lsqrt(V(0.5f) * (s + lsqrt_subnormal(disc)));
+  const V square = V(0.5f) * (s + lproduct(disc, lrsqrt(disc)));
+  return lproduct(square, lrsqrt(square));
 }
 
 // Conserved state and normal flux of a normal-frame primitive state; returns p_T.
@@ -133,7 +130,7 @@ __device__ __forceinline__ void hlld_front_lr(const float (&L)[7], const float (
   for (int c = 0; c < 7; ++c) w[c] = F2(L[c], Rt[c]);
   const L1 vl = L[1], vr = Rt[1];
   const F2 cf2 = fast_speed_l<F2>(w[0], w[4], F2(bn), w[5], w[6], F2(gamma));
-  const L1 cf = lmax(L1(cf2.v.x), L1(cf2.v.y));
+  const L1 cf = max_nan(cf2.v.x, cf2.v.y);
   o.sl = lmin(vl, vr) - cf;
   o.sr = lmax(vl, vr) + cf;
   const L1 bn2 = L1(bn) * L1(bn);
