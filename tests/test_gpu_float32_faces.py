@@ -124,3 +124,20 @@ def test_faces_agree_with_float64(unit, field, speed, limiter):
     for want, got, scale in zip(*results, scales, strict=True):
         assert np.isfinite(got).all()
         assert np.abs(got - want).max() <= bound * scale
+
+
+@pytest.mark.parametrize("ndim", [2, 3])
+def test_the_stable_step_in_units_of_small_speeds(ndim):
+    """Speeds of 1e-10: the discriminants (6e-40) keep 18 bits, their roots 2e-6, the step half
+    of that of its fast speed; 1e-5 with the float32 rounding around them."""
+    from wellbalanced_b200 import MHD2D, MHD3D
+    from wellbalanced_b200.mesh import AMRHierarchy
+
+    unit = 2.0**-33
+    steps = []
+    for precision in (64, 32):
+        mesh = AMRHierarchy((20, 12, 9)[:ndim], periodic=(True,) * ndim)
+        model = (MHD2D if ndim == 2 else MHD3D)(mesh, precision=precision)
+        model.set_state(lambda x, *y: 1.0 + 0.3 * np.sin(6.0 * x), (0.3 * unit, -0.2 * unit, 0.1 * unit), 0.8 * unit**2)
+        steps.append(model.stable_step())
+    assert abs(steps[1] - steps[0]) <= 1e-5 * steps[0]
