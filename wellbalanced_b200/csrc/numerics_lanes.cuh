@@ -20,7 +20,7 @@ namespace wb {
 // roots 6, first-order fallback 12, star states 10, sign 3, region selection 12). They have the
 // bits of the plain selection where no operand or product is subnormal or NaN (a NaN
 // difference, of a cell reported as bad, leaves the slope to the other one). B200: a stage of
-// the 256^3 box 1.98 ms with those, 1.74 now; of 512 2D instances of 32^2 to 256^2 cells, 0.90
+// the 256^3 box 1.98 ms with those, 1.75 now; of 512 2D instances of 32^2 to 256^2 cells, 0.90
 // and 0.81 ms.
 
 // sqrt(x) of a density as x rsqrt(x); x below the smallest normal counts as that, so the root of
